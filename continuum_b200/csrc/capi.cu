@@ -227,6 +227,35 @@ int validate_flat(const cc::FlatScene& f) {
   return CC_OK;
 }
 
+// Whether an in-order walk of a flat scene's own hierarchies could need more
+// than the walk's 64 stack entries (the hierarchies this library builds halve
+// their items at every node and stay far below). A popped node's children
+// take its entry and the next; a triangle hierarchy's right child is popped
+// first, an object node's nearer one. Children follow their parents.
+bool deeper_than_stack(const cc::FlatScene& f) {
+  constexpr uint32_t kMost = 64;
+  auto cap = [](uint32_t v) { return std::min(v, kMost + 1); };
+  std::vector<uint32_t> tree(f.blas.size(), 0), object(f.nodes.size(), 0);
+  for (size_t i = f.blas.size(); i-- > 0;) {
+    const cc::NodeGpu& n = f.blas[i];
+    if (n.info[1] == 0) tree[i] = cap(std::max({2u, tree[n.info[0]], 1u + tree[n.info[0] + 1]}));
+  }
+  for (size_t i = f.nodes.size(); i-- > 0;) {
+    const cc::NodeGpu& n = f.nodes[i];
+    if (n.info[1] == 0) {
+      object[i] = cap(std::max({2u, 1u + object[n.info[0]], 1u + object[n.info[0] + 1]}));
+      continue;
+    }
+    // A leaf's meshes: two entries each, the trees above them.
+    for (uint32_t k = n.info[0]; k < n.info[0] + n.info[1]; ++k) {
+      if (f.items[k] >= f.nmeshes) continue;
+      const uint32_t root = f.ranges[4 * (size_t)f.items[k] + 2];
+      if (root != CC_NONE) object[i] = std::max(object[i], cap(2 * n.info[1] + tree[root]));
+    }
+  }
+  return !object.empty() && object[0] > kMost;
+}
+
 int threads_for_build() {
   unsigned n = std::thread::hardware_concurrency();
   return n ? (int)std::min(n, 32u) : 4;
@@ -348,6 +377,7 @@ int cc_scene_upload(cc_context* ctx, const cc_flat_scene* fl, cc_scene** out) {
     f.xforms.assign(fl->xforms, fl->xforms + (size_t)fl->nxforms * 16);
   }
   int rc = validate_flat(f);
+  if (!rc) s->deep = deeper_than_stack(f);
   if (!rc) rc = set_device(ctx);
   if (!rc) rc = upload_scene(s);
   if (rc) {

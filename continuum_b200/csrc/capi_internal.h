@@ -106,6 +106,7 @@ struct cc_scene {
   // CC_BACK_FACING: each triangle's slot on the device, uploaded on first use.
   uint32_t* tri_slot = nullptr;
   uint64_t bytes = 0;
+  bool deep = false;  // DevScene::deep
   cc::DevScene dev() const {
     cc::DevScene s;
     s.tris = tris;
@@ -117,6 +118,7 @@ struct cc_scene {
     s.xforms = xforms;
     s.blas_cov = blas_cov;
     s.obj_cov = obj_cov;
+    s.deep = deep ? 1u : 0u;
     return s;
   }
 };

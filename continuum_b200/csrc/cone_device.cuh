@@ -59,6 +59,10 @@ struct DevScene {
   // the scene has none on the device.
   const float* blas_cov;
   const float* obj_cov;
+  // A walk of some mesh could need more than the 64 entries of the in-order
+  // walk's stack (a flat scene's own hierarchies): its trees are walked in
+  // order, which flags such a walk.
+  uint32_t deep;
 };
 
 struct DevLight {
@@ -129,16 +133,6 @@ __device__ __forceinline__ f3 direction(const Cone& c, float s, float t) {  // :
 __device__ __forceinline__ f3 to_local(const Cone& c, f3 p) {  // :208-211
   f3 d = p - c.apex;
   return {dot(c.right, d), dot(c.up, d), dot(c.fwd, d)};
-}
-
-__device__ __forceinline__ bool in_bound(const Cone& c, f3 p, float r) {  // :159-168
-  if (c.bcos < -1.0f) return true;
-  f3 d = p - c.apex;
-  float l = len(d);
-  if (l <= r) return true;
-  float s = r / l;
-  float limit = c.bcos * sqrtf(1.0f - s * s) - c.bsin * s;
-  return dot(c.baxis, d) >= limit * l;
 }
 
 __device__ __forceinline__ void bound_cone(Cone& c, f3 axis) {  // :174-186
@@ -259,33 +253,18 @@ __device__ __forceinline__ f3 rotate_to_object(f3 v, const float4* __restrict__ 
   return mk(r0.x, r0.y, r0.z) * v.x + mk(r1.x, r1.y, r1.z) * v.y + mk(r2.x, r2.y, r2.z) * v.z;
 }
 
-// may_touch_box (:234-255), which is node_cone_test (:519-574) for exact cones.
-// kHorizon: sky cones, whose horizon `horizon` (the receiver's normal, in the
-// cone's space) also culls a box wholly below it (:245); a light cone's
-// horizon is zero (:146-147), which culls nothing, so light cones skip it.
-// kUnrolled: the eight corners side by side (the walk's hot test of a node's
-// children); else one at a time, in a fifth of the code (the tests of a
-// walk's root and of meshes' roots, which run far less often).
-template <bool kHorizon = false, bool kUnrolled = true>
-__device__ __forceinline__ bool may_touch_box(const Cone& c, f3 lo, f3 hi, f3 horizon = f3{0.f, 0.f, 0.f}) {
-  bool far_out = true, near_out = true, out_u0 = true, out_u1 = true, out_v0 = true, out_v1 = true, below = kHorizon;
-#pragma unroll (kUnrolled ? 8 : 1)
-  for (int k = 0; k < 8; ++k) {
-    f3 corner = mk((k & 1) ? hi.x : lo.x, (k & 2) ? hi.y : lo.y, (k & 4) ? hi.z : lo.z);
-    if (c.far_offset - dot(c.fwd, corner) >= 0.0f) far_out = false;
-    if constexpr (kHorizon) {
-      if (dot(horizon, corner - c.apex) >= 0.0f) below = false;
-    }
-    f3 p = to_local(c, corner);
-    if (p.z >= kNear) near_out = false;
-    if (p.x - c.u0 * p.z >= 0.0f) out_u0 = false;
-    if (c.u1 * p.z - p.x >= 0.0f) out_u1 = false;
-    if (p.y - c.v0 * p.z >= 0.0f) out_v0 = false;
-    if (c.v1 * p.z - p.y >= 0.0f) out_v1 = false;
-  }
-  if (far_out || near_out || out_u0 || out_u1 || out_v0 || out_v1 || below) return false;
-  return in_bound(c, (lo + hi) * 0.5f, 0.5f * len(hi - lo));
+__device__ __forceinline__ float min_nan(float a, float b) {  // a not-a-number stays one
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
 }
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+#include "box_test.cuh"
 
 // may_touch (:215-232); kHorizon as in may_touch_box (:220-221).
 template <bool kHorizon = false>
@@ -323,24 +302,24 @@ __device__ __forceinline__ bool may_touch(const Cone& c, f3 v0, f3 v1, f3 v2, f3
 constexpr float kFixScale = 16777216.0f;        // 2^24
 constexpr float kFixUnit = 1.0f / 16777216.0f;  // 2^-24
 
-template <class Cell>
+template <class Cell, int kStride>
 struct LaneAcc;
 
 // 64-bit cells: no overflow is possible (each add is at most one bin).
-template <>
-struct LaneAcc<unsigned long long> {
-  unsigned long long* base;  // &acc[cone]; cell k at base[32 * k]
+template <int kStride>
+struct LaneAcc<unsigned long long, kStride> {
+  unsigned long long* base;  // &acc[cone]; cell k at base[kStride * k]
   uint32_t span_lo, span_hi; // rows this triangle wrote (the WGSL's span, :758-760)
   uint32_t* overflow;        // unused
   uint32_t bit;
   __device__ __forceinline__ void add(uint32_t cell, float v) {
-    if (cell < (uint32_t)kBins) atomicAdd(base + 32 * cell, (unsigned long long)__float2ll_rn(v * kFixScale));
+    if (cell < (uint32_t)kBins) atomicAdd(base + kStride * cell, (unsigned long long)__float2ll_rn(v * kFixScale));
   }
 };
 
 // 32-bit cells: a signed overflow of any add sets the cone's bit in *overflow.
-template <>
-struct LaneAcc<unsigned int> {
+template <int kStride>
+struct LaneAcc<unsigned int, kStride> {
   unsigned int* base;
   uint32_t span_lo, span_hi;
   uint32_t* overflow;
@@ -348,7 +327,7 @@ struct LaneAcc<unsigned int> {
   __device__ __forceinline__ void add(uint32_t cell, float v) {
     if (cell < (uint32_t)kBins) {
       const int a = __float2int_rn(v * kFixScale);
-      const int old = (int)atomicAdd(base + 32 * cell, (unsigned int)a);
+      const int old = (int)atomicAdd(base + kStride * cell, (unsigned int)a);
       const int sum = (int)((unsigned int)old + (unsigned int)a);
       if (((old ^ sum) & (a ^ sum)) < 0) atomicOr(overflow, bit);
     }
@@ -472,18 +451,28 @@ __device__ __forceinline__ void draw_polygon(Acc& acc, const float2* q, int n, f
   }
 }
 
-// The clipped polygon in bin space, drawn (general path of rasterize,
-// :350-451): far and near clips, then either the projected corners or, for a
-// polygon reaching outside the window, the window square clipped to the
-// planes through the apex and each edge; finally the square's sides.
-// Every loop here stays rolled and each clip has one call site: the walk
-// kernel is bound by instruction fetch, and the unrolled path (1,832
-// instructions against 1,069) made the packet pass 13 % slower.
-// kWeighted: the triangle is drawn with `weight` (tri_weight: a blended or
-// transmissive object's); else whole.
-template <class Acc, bool kWeighted = false>
-static __device__ __noinline__ bool rasterize_general(const Cone& c, Acc& acc, f3 v0, f3 v1, f3 v2, bool far_clip,
-                                                      float weight = 1.0f) {
+// Whether the triangle reaches past the far plane (rasterize's far clip, :356-362).
+__device__ __forceinline__ bool crosses_far(const Cone& c, f3 v0, f3 v1, f3 v2) {
+  const float f0 = c.far_offset - dot(c.fwd, v0);
+  const float f1 = c.far_offset - dot(c.fwd, v1);
+  const float f2 = c.far_offset - dot(c.fwd, v2);
+  return f0 < 0.0f || f1 < 0.0f || f2 < 0.0f;
+}
+
+// The triangle's polygon in bin space (rasterize, :350-451, up to the
+// drawing), in qa or qb (*out); returns its corners, 0 for nothing to draw.
+// `simple` takes the common case only, a triangle wholly inside the window
+// between the near and far planes, whose three corners are projected, and
+// returns -1 for every other. Else: far and near clips, then either the
+// projected corners or, for a polygon reaching outside the window, the window
+// square clipped to the planes through the apex and each edge; finally the
+// square's sides. Every loop here stays rolled, each clip has one call site
+// and both cases share the code: the walk kernel is bound by instruction
+// fetch.
+__device__ __forceinline__ int bin_polygon(const Cone& c, f3 v0, f3 v1, f3 v2, bool simple, float2* qa, float2* qb,
+                                           float2** out) {
+  const bool far_clip = crosses_far(c, v0, v1, v2);
+  if (simple && far_clip) return -1;
   f3 pa[kPolyCap], pb[kPolyCap];
   pa[0] = v0;
   pa[1] = v1;
@@ -511,15 +500,15 @@ static __device__ __noinline__ bool rasterize_general(const Cone& c, Acc& acc, f
       if (v.x < c.u0 * v.z || v.x > c.u1 * v.z || v.y < c.v0 * v.z || v.y > c.v1 * v.z) all_in_window = false;
     }
   }
-  if (n < 3) return false;
+  if (n < 3) return 0;
   const float su = float(kGrid) / (c.u1 - c.u0);
   const float sv = float(kGrid) / (c.v1 - c.v0);
   const float g = float(kGrid);
-  float2 qa[kPolyCap], qb[kPolyCap];
   float2* q = qa;
   float2* q2 = qb;
   int m;
   const bool projected = all_near_ok && all_in_window;
+  if (simple && !projected) return -1;
   float side = 1.0f;
   if (projected) {
     m = n;
@@ -528,7 +517,7 @@ static __device__ __noinline__ bool rasterize_general(const Cone& c, Acc& acc, f
   } else {
     f3 l0 = to_local(c, v0), l1 = to_local(c, v1), l2 = to_local(c, v2);
     float d = dot(l0, cross(l1, l2));
-    if (d == 0.0f) return false;
+    if (d == 0.0f) return 0;
     side = d > 0.0f ? 1.0f : -1.0f;
     m = 4;
     q[0] = make_float2(0.f, 0.f);
@@ -568,6 +557,7 @@ static __device__ __noinline__ bool rasterize_general(const Cone& c, Acc& acc, f
       for (int j = 0; j < m; ++j)
         if (q[j].x < 0.f || q[j].y < 0.f || q[j].x > g || q[j].y > g) inside = false;
       if (inside) break;
+      if (simple) return -1;
       stage = 2;
       i = 0;
       continue;
@@ -583,70 +573,8 @@ static __device__ __noinline__ bool rasterize_general(const Cone& c, Acc& acc, f
     q = q2;
     q2 = t;
   }
-  if (m < 3) return false;
-  draw_polygon(acc, q, m, kWeighted ? weight : 1.0f);
-  return true;
-}
-
-// Whether the triangle reaches past the far plane (rasterize's far clip, :356-362).
-__device__ __forceinline__ bool crosses_far(const Cone& c, f3 v0, f3 v1, f3 v2) {
-  const float f0 = c.far_offset - dot(c.fwd, v0);
-  const float f1 = c.far_offset - dot(c.fwd, v1);
-  const float f2 = c.far_offset - dot(c.fwd, v2);
-  return f0 < 0.0f || f1 < 0.0f || f2 < 0.0f;
-}
-
-// rasterize (:350-451), its common case: a triangle wholly inside the window
-// between the near and far planes projects its three corners and draws them
-// from registers. Returns false, having drawn nothing, for every other
-// triangle: those take rasterize_general.
-template <class Acc>
-__device__ __forceinline__ bool rasterize_fast(const Cone& c, Acc& acc, f3 v0, f3 v1, f3 v2, float weight = 1.0f) {
-  if (!crosses_far(c, v0, v1, v2)) {
-    f3 p0 = to_local(c, v0), p1 = to_local(c, v1), p2 = to_local(c, v2);
-    auto in_win = [&](f3 v) {
-      return v.z >= kNear && !(v.x < c.u0 * v.z || v.x > c.u1 * v.z || v.y < c.v0 * v.z || v.y > c.v1 * v.z);
-    };
-    if (in_win(p0) && in_win(p1) && in_win(p2)) {
-      const float su = float(kGrid) / (c.u1 - c.u0);
-      const float sv = float(kGrid) / (c.v1 - c.v0);
-      const float g = float(kGrid);
-      // The corners projected in turn (one site for each division).
-      float ax = 0.f, ay = 0.f, bx = 0.f, by = 0.f, cx = 0.f, cy = 0.f;
-      f3 pk = p0;
-#pragma unroll 1
-      for (int k = 0; k < 3; ++k) {
-        ax = bx;
-        ay = by;
-        bx = cx;
-        by = cy;
-        cx = (pk.x / pk.z - c.u0) * su;
-        cy = (pk.y / pk.z - c.v0) * sv;
-        pk = k == 0 ? p1 : p2;
-      }
-      bool inside = ax >= 0.f && ay >= 0.f && ax <= g && ay <= g && bx >= 0.f && by >= 0.f && bx <= g &&
-                    by <= g && cx >= 0.f && cy >= 0.f && cx <= g && cy <= g;
-      if (inside) {
-        // The three edges from one call site (a rolled loop keeps the hot
-        // code small enough for the instruction caches).
-#pragma unroll 1
-        for (int e = 0; e < 3; ++e) {
-          const float sx = e == 0 ? ax : (e == 1 ? bx : cx), sy = e == 0 ? ay : (e == 1 ? by : cy);
-          const float tx = e == 0 ? bx : (e == 1 ? cx : ax), ty = e == 0 ? by : (e == 1 ? cy : ay);
-          draw_edge(acc, sx, sy, tx, ty, weight);
-        }
-        return true;
-      }
-    }
-  }
-  return false;
-}
-
-// rasterize (:350-451): the common case, else the general path.
-template <class Acc>
-__device__ __forceinline__ bool rasterize(const Cone& c, Acc& acc, f3 v0, f3 v1, f3 v2) {
-  if (rasterize_fast(c, acc, v0, v1, v2)) return true;
-  return rasterize_general(c, acc, v0, v1, v2, crosses_far(c, v0, v1, v2));
+  *out = q;
+  return m < 3 ? 0 : m;
 }
 
 // ---- integration --------------------------------------------------------------

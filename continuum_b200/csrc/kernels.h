@@ -9,17 +9,34 @@
 namespace cc {
 
 constexpr int kWarpsPerBlock = 2;
-// Resident blocks per SM the shared memory allows. Passes that keep each
-// cone's coverages in thread-local memory (the split path's, exact sky
-// cones'): the packet pass (32-bit accumulator cells, 22 KB per block) fits
-// 8, the solo pass (64-bit cells, 38 KB) 5; prefiltering sky cones, whose
-// walk needs more registers, 6 and 5. Prefiltering light cones keep them in
-// shared memory: 5 and 4.
+// Cones a warp walks together at most (results do not depend on it). Light
+// cones' tree walk takes its (cone, node) pairs from all of a packet's cones,
+// so a packet of 16 keeps the lanes as busy as one of 32, with half the shared
+// memory and half the time of the heaviest packet, which ends the pass: 32, 16
+// and 8 cones took 41.3, 40.2 and 45.3 ms on 3.69 M cones over 3.07 M
+// triangles and 10.7, 7.2 and 5.9 ms on 229 k cones. Sky and prefiltering
+// cones, which integrate their masks in the walk kernel, a lane each, keep 32
+// (exact sky cones: 6.4 ms, 8.3 with 16).
+constexpr uint32_t kPacketCones = 16;
+constexpr uint32_t kFusedPacketCones = 32;
+// `fused`: sky or prefiltering cones.
+constexpr uint32_t packet_cones(uint32_t points_per_warp, bool fused = false) {
+  const uint32_t most = fused ? kFusedPacketCones : kPacketCones;
+  return points_per_warp < most ? points_per_warp : most;
+}
+// Resident blocks per SM. Passes that keep each cone's coverages in
+// thread-local memory (the split path's, exact sky cones') take 8: 128
+// registers a thread, and 16 KB of shared memory per block in the packet pass
+// (27 KB for sky cones; the solo pass holds one cone's cells, 6 KB). 10 and 12
+// blocks (96 and 80 registers, with spills) ran the same: instruction fetch,
+// not the warps in flight, is the bound. Prefiltering sky cones, whose walk needs more
+// registers, take 6. Prefiltering light cones keep their coverages in shared
+// memory: 5.
 constexpr int kBlocksPerSm = 8;
-constexpr int kSoloBlocksPerSm = 5;
+constexpr int kSoloBlocksPerSm = 8;
 constexpr int kFusedBlocksPerSm = 5;
-constexpr int kFusedSoloBlocksPerSm = 4;
-constexpr int kSkySplatBlocksPerSm = 6;  // prefiltering sky cones' packet pass (thread-local coverages)
+constexpr int kFusedSoloBlocksPerSm = 5;
+constexpr int kSkySplatBlocksPerSm = 6;  // prefiltering sky cones' passes (thread-local coverages)
 
 struct DevQuery {
   const float4* receivers;  // 2 per point: point, normal

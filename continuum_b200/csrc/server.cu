@@ -328,7 +328,7 @@ struct JobGroup {
 // `status` (kCounterWords). Returns false once it has abandoned the launch.
 bool enqueue_group(cc_server* s, Slot& slot, JobGroup& g, bool splat, cc::JobGpu* staging, uint32_t* status) {
   cudaStream_t st = slot.stream;
-  const uint32_t pw = s->opt.points_per_warp;
+  const uint32_t pw = cc::packet_cones(s->opt.points_per_warp, splat);
   cudaError_t e = cudaSuccess;
   std::memcpy(staging, g.jobs.data(), g.jobs.size() * sizeof(cc::JobGpu));
   const uint64_t sort_bytes = cc::batch_order_scratch_bytes(g.points);
@@ -407,7 +407,6 @@ bool enqueue_group(cc_server* s, Slot& slot, JobGroup& g, bool splat, cc::JobGpu
 void launch(cc_server* s, Slot& slot) {
   cudaStream_t st = slot.stream;
   JobGroup exact, splat;  // exact cones; prefiltering cones
-  const uint32_t pw = s->opt.points_per_warp;
   cc_options d;
   cc_options_default(&d);
   for (Request* r : slot.reqs) {
@@ -458,7 +457,8 @@ void launch(cc_server* s, Slot& slot) {
           j.lo[k] = sc->flat.nodes[0].lo[k];
           j.hi[k] = sc->flat.nodes[0].hi[k];
         }
-      (q.prefilter > 0.0f ? splat : exact).add(j, P, pw);
+      const bool prefilter = q.prefilter > 0.0f;
+      (prefilter ? splat : exact).add(j, P, cc::packet_cones(s->opt.points_per_warp, prefilter));
       ++t;
     }
   }

@@ -106,7 +106,7 @@ __device__ __forceinline__ float box_silhouette(const Cone& c, f3 lo, f3 hi, f3*
 // draw, 2 if splatted and drawn into `acc`, 3 if the cone must descend.
 // kHorizon: sky cones (their horizon culls a box wholly below it).
 template <bool kHorizon, class Acc>
-__device__ __noinline__ int node_cone_test(const Cone& c, f3 horizon, Acc& acc, const float* __restrict__ cov, f3 lo,
+__device__ __forceinline__ int node_cone_test(const Cone& c, f3 horizon, Acc& acc, const float* __restrict__ cov, f3 lo,
                                            f3 hi, float prefilter) {
   const float g = float(kGrid);
   float2 pts[8];
@@ -148,6 +148,42 @@ __device__ __noinline__ int node_cone_test(const Cone& c, f3 horizon, Acc& acc, 
   const float alpha = node_front_area(cov, v) / silhouette;
   if (alpha <= 0.0f) return 1;
   return draw_hull(acc, pts, alpha) ? 2 : 1;
+}
+
+// node_cone_test's first answer from box_verdict and two opposite corners:
+// 0 (cannot touch), 3 (descend), or 4: ask node_cone_test. A node that
+// touches is descended into when some corner lies before the apex or past the
+// far plane, or when the box is wider in the cone than `prefilter` bins; of
+// the corners farthest apart along the window's right (and up) axis, the
+// projections' distance is a lower bound of that width. Every comparison
+// leaves box_verdict's slack, so the answer is node_cone_test's.
+template <bool kHorizon>
+__device__ __forceinline__ int quick_node_test(const Cone& c, const BoxTest& t, f3 lo, f3 hi, f3 horizon,
+                                               float prefilter) {
+  const int v = box_verdict<kHorizon>(c, t, lo, hi, horizon);
+  if (v != 1) return v == 0 ? 0 : 4;
+  const f3 a = lo - c.apex, b = hi - c.apex;
+  const f3 m = a + b, e = b - a;
+  const float reach = (fabsf(m.x) + e.x) + (fabsf(m.y) + e.y) + (fabsf(m.z) + e.z);
+  const float slack = kBoxSlack * reach;
+  const float fm = fdot(c.fwd, m, 0.0f), fe = fdot_abs(c.fwd, e, 0.0f);
+  if (fm - fe < -slack) return 3;
+  if (t.far_rel - fm - fe < -(2.0f * __fmaf_rn(kBoxSlack, t.world, slack) + kBoxSlack * fabsf(c.far_offset))) return 3;
+  bool wide = false;
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    const f3 axis = k ? c.up : c.right;
+    const float x = fdot(axis, m, 0.0f), w = fdot_abs(axis, e, 0.0f);
+    const float z = fdot(c.fwd, mk(copysignf(e.x, axis.x), copysignf(e.y, axis.y), copysignf(e.z, axis.z)), 0.0f);
+    const float z0 = fm - z, z1 = fm + z, least = fminf(z0, z1);
+    if (!(least > 64.0f * slack)) continue;
+    const float q0 = __fdividef(x - w, z0), q1 = __fdividef(x + w, z1);
+    const float side = k ? c.v1 - c.v0 : c.u1 - c.u0;
+    if (fabsf(q1 - q0) - __fdividef(4.0f * slack * (1.0f + fabsf(q0) + fabsf(q1)), least) >
+        1.001f * prefilter * side * (1.0f / float(kGrid)))
+      wide = true;
+  }
+  return wide ? 3 : 4;
 }
 
 // splat_object_node (:1096-1150) up to the drawing: whether object node lo..hi

@@ -17,12 +17,24 @@ namespace cc {
 static __constant__ float c_disk[kBins];  // DISK (mask_cones.wgsl:888-897), uploaded by the host
 
 constexpr int kStack = 64;         // entries; the reference's is 48 (mask_cones.wgsl:111)
-constexpr int kConeFields = 17;    // apex, right, up, forward, window, far offset
+constexpr int kConeFields = 22;    // apex, right, up, forward, window, far offset, bounding cone
 // Pairs passed to rasterization wait in a per-warp queue until 32 are ready:
 // a cull round adds at most 32 to at most 31 waiting. Pairs that need the
 // general clip path wait in a second queue of the same size.
 constexpr int kQueueCap = 64;
-constexpr uint32_t kQueueOwnerShift = 26;  // entry: cone lane << 26 | triangle slot (< 2^26)
+constexpr uint32_t kQueueOwnerShift = 26;  // entry: cone lane << 26 | triangle slot or node (< 2^26)
+constexpr uint32_t kQueueIndexMask = (1u << kQueueOwnerShift) - 1u;
+// The tree walk's stack of (cone, node) pairs. A step takes at most 32 pairs
+// and leaves at most two for each, and takes one alone once fewer than kStack
+// entries are left, which holds a whole depth-first descent (scenes whose
+// trees could need more are walked in order: DevScene::deep).
+constexpr int kPairCap = 256;
+// Prefiltering cones' pairs: as many again stay free for the nodes that wait
+// in `splats` (64 entries: a step adds at most 32 to at most 31).
+constexpr int kSplatPairCap = 384;
+constexpr int kSplatCap = 64;
+// Pairs of a cone and a leaf it reaches: a step adds at most 64 to at most 31.
+constexpr int kLeafCap = 96;
 // Both queues' lengths in one word: fast queue in the low byte, general
 // queue in the next (each below 32 between rounds).
 __device__ __forceinline__ uint32_t fast_len(uint32_t q) { return q & 255u; }
@@ -40,35 +52,41 @@ __device__ __forceinline__ uint32_t queue_lens(uint32_t fast, uint32_t general) 
 // Weighted: instanced scenes, whose placed objects may be alpha-blended or
 // transmissive (the transform's `clear`): triangles are drawn with the
 // current object's weight; other launches draw every triangle whole.
-template <class CellT, bool Sky, bool SmemCov, bool Back = false, bool Weighted = false>
+// Cones: those a warp walks together at most (one in the solo pass).
+template <class CellT, bool Sky, bool SmemCov, bool Back = false, bool Weighted = false, int Cones = 32,
+          bool Splat = false>
 struct WarpShared {
   using Cell = CellT;
   static constexpr bool kSky = Sky;
   static constexpr bool kSmemCov = SmemCov;
   static constexpr bool kBack = Back;
   static constexpr bool kWeighted = Weighted;
-  Cell acc[kBins * 32];                 // each cone's accumulator (fixed point, units of kFixUnit)
-  float cone[kConeFields * 32];         // each cone's frame, field-major; the integration's scratch after the walk
-  uint32_t span_lo[32], span_hi[32];    // each cone's accumulator rows written (the WGSL's span)
+  static constexpr bool kSplat = Splat;
+  static constexpr int kPairs = Splat ? kSplatPairCap : kPairCap;
+  static constexpr int kCones = Cones;
+  static constexpr int kConeWords = kConeFields * kCones;
+  Cell acc[kBins * kCones];             // each cone's accumulator (fixed point, units of kFixUnit)
+  // Each cone's frame, field-major; the integration's scratch after the walk.
+  float cone[SmemCov && kConeWords < 388 ? 388 : (kConeWords + 3) / 4 * 4];
+  uint32_t span_lo[kCones + 3 & ~3], span_hi[kCones + 3 & ~3];  // each cone's accumulator rows written (the WGSL's span)
   uint32_t queue[kQueueCap];            // (cone, triangle) pairs that passed the cull, waiting to be rasterized
   uint32_t general[kQueueCap];          // pairs that need rasterize's general path, waiting for it
   uint32_t overflow[4];                 // word 0: cones whose 32-bit accumulation overflowed in the current mesh
-  float horizon[Sky ? 3 * 32 : 4];      // sky cones: each cone's horizon, field-major
+  float horizon[Sky ? (3 * kCones + 3 & ~3) : 4];  // sky cones: each cone's horizon, field-major
   float cov[SmemCov ? kBins * 32 : 4];  // each cone's 64 coverages, bin-major, lane innermost
   // The placed object being walked (Weighted): its triangles' weight and its
   // transmission (add_mesh_coverage_if's tri_weight / tri_transmit /
   // tri_volume, :725-741); weight 1 and no transmission elsewhere.
   float object_weight, object_transmit;
   uint32_t object_volume, object_pad;
+  // The tree walk: pairs (cone, left child) to test, pairs (cone, leaf) to
+  // cull, the work each cone's cap leaves it, and the nodes it visited.
+  uint32_t pairs[kPairs];
+  uint32_t splats[Splat ? kSplatCap : 4];  // prefiltering cones: pairs for node_cone_test
+  uint32_t leaves[kLeafCap];
+  int budget[kCones + 3 & ~3];
+  uint32_t visited[kCones + 3 & ~3];
 };
-static_assert(sizeof(WarpShared<unsigned int, false, true>) % 16 == 0, "warp shared block keeps 16-byte alignment");
-static_assert(sizeof(WarpShared<unsigned long long, false, true>) % 16 == 0, "warp shared block keeps 16-byte alignment");
-static_assert(sizeof(WarpShared<unsigned int, true, true>) % 16 == 0, "warp shared block keeps 16-byte alignment");
-static_assert(sizeof(WarpShared<unsigned int, false, false>) % 16 == 0, "warp shared block keeps 16-byte alignment");
-template <bool kSky, bool kSmemCov, bool kBack = false, bool kWeighted = false>
-using NarrowShared = WarpShared<unsigned int, kSky, kSmemCov, kBack, kWeighted>;
-template <bool kSky, bool kSmemCov, bool kBack = false, bool kWeighted = false>
-using WideShared = WarpShared<unsigned long long, kSky, kSmemCov, kBack, kWeighted>;
 // The shared memory of a kernel variant's warps, and the blocks per SM it
 // fits. Prefiltering light cones integrate in the walk kernel, reading every
 // lane's coverages (warp_blocked): their table stays in shared memory. The
@@ -79,26 +97,28 @@ using WideShared = WarpShared<unsigned long long, kSky, kSmemCov, kBack, kWeight
 template <bool kSky, bool kSplat>
 constexpr bool smem_cov() { return kSplat && !kSky; }
 template <bool kWide, bool kSky, bool kSplat, bool kBack = false, bool kInst = false>
-using KernelShared = typename std::conditional<kWide, WideShared<kSky, smem_cov<kSky, kSplat>(), kBack, kInst>,
-                                               NarrowShared<kSky, smem_cov<kSky, kSplat>(), kBack, kInst>>::type;
+using KernelShared = typename std::conditional<
+    kWide, WarpShared<unsigned long long, kSky, smem_cov<kSky, kSplat>(), kBack, kInst, 1, kSplat>,
+    WarpShared<unsigned int, kSky, smem_cov<kSky, kSplat>(), kBack, kInst,
+               (int)(kSky || kSplat ? kFusedPacketCones : kPacketCones), kSplat>>::type;
 constexpr int resident_blocks_for(bool wide, bool sky, bool splat) {
   return (splat && !sky) ? (wide ? kFusedSoloBlocksPerSm : kFusedBlocksPerSm)
-                         : (wide ? kSoloBlocksPerSm : (splat ? kSkySplatBlocksPerSm : kBlocksPerSm));
+                         : (splat ? kSkySplatBlocksPerSm : (wide ? kSoloBlocksPerSm : kBlocksPerSm));
 }
 template <bool kWide, bool kSky, bool kSplat>
 constexpr int resident_blocks() { return resident_blocks_for(kWide, kSky, kSplat); }
-// Per SM (228 KB): 8 x 22.8 KB and 5 x 38.9 KB with thread-local coverages,
-// 5 x 38.9 KB and 4 x 55.3 KB with shared ones, 1 KB reserved per block.
-static_assert(8 * (kWarpsPerBlock * sizeof(KernelShared<false, false, false>) + 1024) <= 233472, "split packet pass");
-static_assert(5 * (kWarpsPerBlock * sizeof(KernelShared<true, false, false>) + 1024) <= 233472, "split solo pass");
-static_assert(8 * (kWarpsPerBlock * sizeof(KernelShared<false, true, false>) + 1024) <= 233472, "sky packet pass");
-static_assert(5 * (kWarpsPerBlock * sizeof(KernelShared<true, true, false>) + 1024) <= 233472, "sky solo pass");
-static_assert(5 * (kWarpsPerBlock * sizeof(KernelShared<false, false, true>) + 1024) <= 233472, "prefiltering packet pass");
-static_assert(4 * (kWarpsPerBlock * sizeof(KernelShared<true, false, true>) + 1024) <= 233472, "prefiltering solo pass");
-static_assert(6 * (kWarpsPerBlock * sizeof(KernelShared<false, true, true>) + 1024) <= 233472, "prefiltering sky packet pass");
-static_assert(5 * (kWarpsPerBlock * sizeof(KernelShared<true, true, true>) + 1024) <= 233472, "prefiltering sky solo pass");
+// Per SM (228 KB), 1 KB of it reserved per block.
+template <bool kWide, bool kSky, bool kSplat>
+constexpr bool shared_fits() {
+  return sizeof(KernelShared<kWide, kSky, kSplat>) % 16 == 0 &&  // each warp's block keeps 16-byte alignment
+         resident_blocks<kWide, kSky, kSplat>() *
+             (kWarpsPerBlock * sizeof(KernelShared<kWide, kSky, kSplat>) + 1024) <= 233472;
+}
+static_assert(shared_fits<false, false, false>() && shared_fits<true, false, false>(), "split passes");
+static_assert(shared_fits<false, true, false>() && shared_fits<true, true, false>(), "sky passes");
+static_assert(shared_fits<false, false, true>() && shared_fits<true, false, true>(), "prefiltering passes");
+static_assert(shared_fits<false, true, true>() && shared_fits<true, true, true>(), "prefiltering sky passes");
 constexpr uint32_t kStatusAccOverflow = 32u;
-static_assert(kConeFields * 32 >= 387, "the integration scratch fits in the cone table");
 
 // A stack entry packed in one word: its kind in the top 2 bits (an
 // object-hierarchy node, a triangle-hierarchy node, or a mesh's resolve
@@ -166,6 +186,7 @@ struct LaneState {
   bool independent;  // sky cones: meshes combine as independent occluders (else by the maximum)
   f3 horizon;        // sky cones: the horizon in the space of the object being walked (the world's elsewhere)
   f3 world_horizon;  // sky cones in instanced scenes: the horizon in world space
+  const ConeRecord* rec;  // the split path: the cone's record
   // The cone's coverage of bin b.
   __device__ __forceinline__ float& cov_at(int b) { return cov[(WS::kSmemCov ? 32 : 1) * b]; }
 };
@@ -174,71 +195,112 @@ __device__ __forceinline__ f3 node_lo(float4 a) { return mk(a.x, a.y, a.z); }
 
 template <class WS>
 __device__ __forceinline__ void store_cone(WS* ws, const Cone& c, int lane) {
+  if (WS::kCones < 32 && lane >= WS::kCones) return;
   float* t = ws->cone + lane;
-  const float f[kConeFields] = {c.apex.x, c.apex.y, c.apex.z, c.right.x, c.right.y, c.right.z, c.up.x, c.up.y,
-                                c.up.z,   c.fwd.x,  c.fwd.y,  c.fwd.z,   c.u0,      c.v0,      c.u1,   c.v1,
-                                c.far_offset};
+  const float f[kConeFields] = {c.apex.x, c.apex.y, c.apex.z, c.right.x, c.right.y, c.right.z,  c.up.x,    c.up.y,
+                                c.up.z,   c.fwd.x,  c.fwd.y,  c.fwd.z,   c.u0,      c.v0,       c.u1,      c.v1,
+                                c.far_offset, c.baxis.x, c.baxis.y, c.baxis.z, c.bcos, c.bsin};
 #pragma unroll
-  for (int k = 0; k < kConeFields; ++k) t[32 * k] = f[k];
+  for (int k = 0; k < kConeFields; ++k) t[WS::kCones * k] = f[k];
 }
 
 // Sky cones: the lane's horizon beside its cone (the cull reads both).
 template <class WS>
 __device__ __forceinline__ void store_horizon(WS* ws, f3 h, int lane) {
   if constexpr (WS::kSky) {
+    if (WS::kCones < 32 && lane >= WS::kCones) return;
     ws->horizon[lane] = h.x;
-    ws->horizon[32 + lane] = h.y;
-    ws->horizon[64 + lane] = h.z;
+    ws->horizon[WS::kCones + lane] = h.y;
+    ws->horizon[2 * WS::kCones + lane] = h.z;
   }
+}
+template <class WS>
+__device__ __forceinline__ f3 load_horizon(const WS* ws, int owner) {
+  if constexpr (WS::kSky)
+    return mk(ws->horizon[owner], ws->horizon[WS::kCones + owner], ws->horizon[2 * WS::kCones + owner]);
+  return mk(0.f, 0.f, 0.f);
 }
 
 template <class WS>
 __device__ __forceinline__ Cone load_cone(const WS* ws, int owner) {
   const float* t = ws->cone + owner;
+  constexpr int k = WS::kCones;
   Cone c;
-  c.apex = mk(t[0], t[32], t[64]);
-  c.right = mk(t[96], t[128], t[160]);
-  c.up = mk(t[192], t[224], t[256]);
-  c.fwd = mk(t[288], t[320], t[352]);
-  c.u0 = t[384];
-  c.v0 = t[416];
-  c.u1 = t[448];
-  c.v1 = t[480];
-  c.far_offset = t[512];
-  c.baxis = mk(0.f, 0.f, 0.f);
-  c.bcos = c.bsin = 0.f;
+  c.apex = mk(t[0], t[k], t[2 * k]);
+  c.right = mk(t[3 * k], t[4 * k], t[5 * k]);
+  c.up = mk(t[6 * k], t[7 * k], t[8 * k]);
+  c.fwd = mk(t[9 * k], t[10 * k], t[11 * k]);
+  c.u0 = t[12 * k];
+  c.v0 = t[13 * k];
+  c.u1 = t[14 * k];
+  c.v1 = t[15 * k];
+  c.far_offset = t[16 * k];
+  c.baxis = mk(t[17 * k], t[18 * k], t[19 * k]);
+  c.bcos = t[20 * k];
+  c.bsin = t[21 * k];
   return c;
 }
 
-// The tests of cover_triangle (:594-616) for one (triangle, cone) pair: back
+// A cone as cone_setup_kernel set it up.
+__device__ __forceinline__ Cone record_cone(const ConeRecord& rec) {
+  Cone c;
+  c.apex = mk(rec.a.x, rec.a.y, rec.a.z);
+  c.far_offset = rec.a.w;
+  c.right = mk(rec.b.x, rec.b.y, rec.b.z);
+  c.u0 = rec.b.w;
+  c.up = mk(rec.c.x, rec.c.y, rec.c.z);
+  c.v0 = rec.c.w;
+  c.fwd = mk(rec.d.x, rec.d.y, rec.d.z);
+  c.u1 = rec.d.w;
+  c.baxis = mk(rec.e.x, rec.e.y, rec.e.z);
+  c.v1 = rec.e.w;
+  c.bcos = rec.f.x;
+  c.bsin = rec.f.y;
+  return c;
+}
+
+// An instanced scene's walk: the lane's cone in world space, from its record
+// (22 registers held through the tree walk would be spilled there; sky cones
+// have none).
+template <class WS>
+__device__ __forceinline__ Cone world_cone(const LaneState<WS>& st) {
+  if constexpr (WS::kSky) return st.cone;
+  else return record_cone(*st.rec);
+}
+
+// The four directions of a cone's window corners.
+struct Corners {
+  f3 d00, d10, d01, d11;
+};
+__device__ __forceinline__ Corners corners_of(const Cone& c) {
+  return {direction(c, 0.f, 0.f), direction(c, 1.f, 0.f), direction(c, 0.f, 1.f), direction(c, 1.f, 1.f)};
+}
+
+// The tests of cover_triangle (:594-616) for triangle slot t and cone c: back
 // face, the window-direction test, may_touch. A pair that passes is
 // rasterized.
-template <class WS>
-__device__ __forceinline__ bool pair_survives(const DevScene& s, const WS* ws, int owner, uint32_t t) {
-  const Cone c = load_cone(ws, owner);
-  const f3 v0 = xyz(__ldg(&s.tris[3 * (size_t)t + 0]));
-  const f3 v1 = xyz(__ldg(&s.tris[3 * (size_t)t + 1]));
-  const f3 v2 = xyz(__ldg(&s.tris[3 * (size_t)t + 2]));
+template <bool kSky>
+__device__ __forceinline__ bool pair_survives(const float4* __restrict__ tris, const Cone& c, const Corners& w,
+                                              f3 horizon, uint32_t t) {
+  const f3 v0 = xyz(__ldg(&tris[3 * (size_t)t + 0]));
+  const f3 v1 = xyz(__ldg(&tris[3 * (size_t)t + 1]));
+  const f3 v2 = xyz(__ldg(&tris[3 * (size_t)t + 2]));
   const f3 n = cross(v1 - v0, v2 - v0);
   if (dot(n, c.apex - v0) <= 0.0f) return false;  // faces away (:600)
-  if (dot(n, direction(c, 0.f, 0.f)) >= 0.f && dot(n, direction(c, 1.f, 0.f)) >= 0.f &&
-      dot(n, direction(c, 0.f, 1.f)) >= 0.f && dot(n, direction(c, 1.f, 1.f)) >= 0.f)
+  if (dot(n, w.d00) >= 0.f && dot(n, w.d10) >= 0.f && dot(n, w.d01) >= 0.f && dot(n, w.d11) >= 0.f)
     return false;  // every window direction leaves its plane (:601-606)
-  if constexpr (WS::kSky)
-    return may_touch<true>(c, v0, v1, v2, mk(ws->horizon[owner], ws->horizon[32 + owner], ws->horizon[64 + owner]));
-  else
-    return may_touch(c, v0, v1, v2);
+  return may_touch<kSky>(c, v0, v1, v2, horizon);
 }
 
 template <class WS>
-__device__ __forceinline__ void load_pair(const DevScene& s, const WS* ws, uint32_t e, int& owner, Cone& c,
-                                          f3& v0, f3& v1, f3& v2) {
+__device__ __forceinline__ void load_pair(const float4* __restrict__ tris, const WS* ws, uint32_t e, int& owner,
+                                          Cone& c, f3& v0, f3& v1, f3& v2) {
   owner = (int)(e >> kQueueOwnerShift);
-  const uint32_t t = e & ((1u << kQueueOwnerShift) - 1u);
+  const uint32_t t = e & kQueueIndexMask;
   c = load_cone(ws, owner);
-  v0 = xyz(__ldg(&s.tris[3 * (size_t)t + 0]));
-  v1 = xyz(__ldg(&s.tris[3 * (size_t)t + 1]));
-  v2 = xyz(__ldg(&s.tris[3 * (size_t)t + 2]));
+  v0 = xyz(__ldg(&tris[3 * (size_t)t + 0]));
+  v1 = xyz(__ldg(&tris[3 * (size_t)t + 1]));
+  v2 = xyz(__ldg(&tris[3 * (size_t)t + 2]));
 }
 
 // The weight a (triangle, cone) pair is drawn with: the current object's
@@ -299,52 +361,53 @@ __device__ __forceinline__ void note_span(WS* ws, int owner, const Acc& acc) {
   }
 }
 
-// The general path for general-queue entries first .. first+n (n <= 32),
-// one per lane.
+// Rasterizes `n` (at most 32) pairs, one per lane, each into its cone's
+// accumulator: the last `n` of the queue (of length `queued`) by the common
+// case, the pairs that need the general path joining the general queue, which
+// is run whenever 32 wait (with `n` 0: at once, whatever its length). Returns
+// the general queue's new length (below 32). One body for both cases: the
+// walk is bound by instruction fetch.
 template <class WS>
-__device__ __noinline__ void raster_general(const DevScene& s, WS* ws, uint32_t first, uint32_t n, int lane) {
-  if ((uint32_t)lane < n) {
-    int owner;
-    Cone c;
-    f3 v0, v1, v2;
-    load_pair(s, ws, ws->general[first + lane], owner, c, v0, v1, v2);
-    LaneAcc<typename WS::Cell> acc{ws->acc + owner, 68u, 0u, &ws->overflow[0], 1u << owner};
-    float weight = 1.0f;
-    if constexpr (WS::kWeighted) weight = pair_weight(ws, c, v0, v1, v2);
-    rasterize_general<decltype(acc), WS::kWeighted>(c, acc, v0, v1, v2, crosses_far(c, v0, v1, v2), weight);
-    note_span(ws, owner, acc);
+static __device__ __noinline__ uint32_t raster_pairs(const float4* __restrict__ tris, WS* ws, uint32_t first,
+                                                     uint32_t n, uint32_t general, int lane) {
+  bool simple = n > 0;
+  if (!simple) {
+    n = general;
+    first = general = 0;
   }
-  __syncwarp();
-}
-
-// Rasterizes queue entries first .. first+n (n <= 32), one per lane, each
-// into its cone's accumulator by the common case; pairs that need the
-// general path join the general queue, which is run whenever 32 wait.
-// Returns the general queue's new length (below 32).
-template <class WS>
-__device__ __noinline__ uint32_t raster_queue(const DevScene& s, WS* ws, uint32_t first, uint32_t n,
-                                              uint32_t general, int lane) {
-  bool defer = false;
-  uint32_t e = 0;
-  if ((uint32_t)lane < n) {
-    e = ws->queue[first + lane];
-    int owner;
-    Cone c;
-    f3 v0, v1, v2;
-    load_pair(s, ws, e, owner, c, v0, v1, v2);
-    LaneAcc<typename WS::Cell> acc{ws->acc + owner, 68u, 0u, &ws->overflow[0], 1u << owner};
-    float weight = 1.0f;
-    if constexpr (WS::kWeighted) weight = pair_weight(ws, c, v0, v1, v2);
-    defer = !rasterize_fast(c, acc, v0, v1, v2, weight);
-    note_span(ws, owner, acc);
-  }
-  const uint32_t m = __ballot_sync(0xffffffffu, defer);
-  if (defer) ws->general[general + __popc(m & ((1u << lane) - 1u))] = e;
-  general += __popc(m);
-  __syncwarp();
-  if (general >= 32) {
-    general -= 32;
-    raster_general(s, ws, general, 32, lane);
+#pragma unroll 1
+  while (n > 0) {
+    const uint32_t* src = simple ? ws->queue : ws->general;
+    int m = 0;
+    uint32_t e = 0;
+    if ((uint32_t)lane < n) {
+      e = src[first + lane];
+      int owner;
+      Cone c;
+      f3 v0, v1, v2;
+      load_pair(tris, ws, e, owner, c, v0, v1, v2);
+      float2 qa[kPolyCap], qb[kPolyCap];
+      float2* q = qa;
+      m = bin_polygon(c, v0, v1, v2, simple, qa, qb, &q);
+      if (m > 0) {
+        LaneAcc<typename WS::Cell, WS::kCones> acc{ws->acc + owner, 68u, 0u, &ws->overflow[0], 1u << owner};
+        float weight = 1.0f;
+        if constexpr (WS::kWeighted) weight = pair_weight(ws, c, v0, v1, v2);
+        draw_polygon(acc, q, m, weight);
+        note_span(ws, owner, acc);
+      }
+    }
+    __syncwarp();
+    if (!simple) break;
+    const uint32_t defer = __ballot_sync(0xffffffffu, m < 0);
+    if (m < 0) ws->general[general + __popc(defer & ((1u << lane) - 1u))] = e;
+    general += __popc(defer);
+    __syncwarp();
+    // Then the general queue's last 32, if as many wait.
+    simple = false;
+    n = general >= 32 ? 32 : 0;
+    general -= n;
+    first = general;
   }
   return general;
 }
@@ -358,7 +421,7 @@ __device__ __noinline__ uint32_t raster_queue(const DevScene& s, WS* ws, uint32_
 // `skip` is the lane's cone's own triangle slot (kNoneU: none), which it
 // does not draw; `skips` (warp-uniform) says some lane has one.
 template <class WS>
-__device__ __noinline__ uint32_t cover_leaf(const DevScene& s, WS* ws, uint32_t owners, uint32_t t0,
+__device__ __noinline__ uint32_t cover_leaf(const float4* __restrict__ tris, WS* ws, uint32_t owners, uint32_t t0,
                                             uint32_t nt, uint32_t queues, int lane, uint32_t skip, bool skips) {
   uint32_t queued = fast_len(queues), general = general_len(queues);
   const uint32_t n_owners = __popc(owners);
@@ -379,7 +442,8 @@ __device__ __noinline__ uint32_t cover_leaf(const DevScene& s, WS* ws, uint32_t 
       const uint32_t r = pair - k * n_owners;
       owner = (int)__fns(owners, 0, r + 1);
       t = t0 + k;
-      pass = pair_survives(s, ws, owner, t);
+      const Cone c = load_cone(ws, owner);
+      pass = pair_survives<WS::kSky>(tris, c, corners_of(c), load_horizon(ws, owner), t);
       entry = ((uint32_t)owner << kQueueOwnerShift) | t;
     }
     // The owner's own triangle is not drawn (cover_triangle's cover_skip, :595).
@@ -392,7 +456,7 @@ __device__ __noinline__ uint32_t cover_leaf(const DevScene& s, WS* ws, uint32_t 
     __syncwarp();
     if (queued >= 32) {
       queued -= 32;
-      general = raster_queue(s, ws, queued, 32, general, lane);
+      general = raster_pairs(tris, ws, queued, 32, general, lane);
     }
   }
   return queue_lens(queued, general);
@@ -404,15 +468,18 @@ __device__ __noinline__ uint32_t cover_leaf(const DevScene& s, WS* ws, uint32_t 
 // (1 - (1 - before)(1 - covered), :819-821); then the cells are cleared for
 // the next mesh.
 template <class WS>
+__device__ __forceinline__ void drain_queues(const float4* __restrict__ tris, WS* ws, uint32_t& queued, int lane) {
+  // The mesh's last pairs: the common case, then the general path.
+  uint32_t general = general_len(queued);
+  if (fast_len(queued)) general = raster_pairs(tris, ws, 0, fast_len(queued), general, lane);
+  if (general) raster_pairs(tris, ws, 0, 0, general, lane);
+  queued = 0;
+}
+
+template <class WS>
 __device__ __forceinline__ void resolve_mesh(const DevScene& s, LaneState<WS>& st, int lane, bool splat = false) {
   WS* ws = st.ws;
-  // The mesh's last pairs: the common case, then the general path.
-  uint32_t general = general_len(st.queued);
-  if (fast_len(st.queued)) general = raster_queue(s, ws, 0, fast_len(st.queued), general, lane);
-  if (general) raster_general(s, ws, 0, general, lane);
-  st.queued = 0;
-  const uint32_t lo = ws->span_lo[lane];
-  const uint32_t end = min(ws->span_hi[lane], (uint32_t)kBins);
+  drain_queues(s.tris, ws, st.queued, lane);
   // 32-bit cells: a cone whose adds overflowed in this mesh is walked again
   // with 64-bit cells (its result here is discarded).
   if (sizeof(typename WS::Cell) == 4) {
@@ -420,39 +487,40 @@ __device__ __forceinline__ void resolve_mesh(const DevScene& s, LaneState<WS>& s
     __syncwarp();
     if (lane == 0) ws->overflow[0] = 0u;
   }
-  long long running = 0;
-  for (uint32_t b = lo; b < end; ++b) {
-    typename WS::Cell* cell = &ws->acc[32 * b + lane];
-    if (sizeof(typename WS::Cell) == 4) running += (long long)(int)*cell;
-    else running += (long long)*cell;
-    *cell = 0;
-    float covered = fabsf(__ll2float_rn(running) * kFixUnit);
-    // An object-level splat is combined without the whole-bin snap (:1137).
-    if (splat) covered = fminf(covered, 1.0f);
-    else if (covered >= 1.0f - 1e-5f) covered = 1.0f;
-    if (covered > 1e-6f) {
-      const float before = st.cov_at(b);
-      float after;
-      if constexpr (WS::kSky) {
-        after = st.independent ? 1.0f - (1.0f - before) * (1.0f - fminf(covered, 1.0f))
-                               : fmaxf(before, fminf(covered, 1.0f));
-      } else {
-        after = fmaxf(before, fminf(covered, 1.0f));
+  if (WS::kCones == 32 || lane < WS::kCones) {
+    const uint32_t lo = ws->span_lo[lane];
+    const uint32_t end = min(ws->span_hi[lane], (uint32_t)kBins);
+    long long running = 0;
+    for (uint32_t b = lo; b < end; ++b) {
+      typename WS::Cell* cell = &ws->acc[WS::kCones * b + lane];
+      if (sizeof(typename WS::Cell) == 4) running += (long long)(int)*cell;
+      else running += (long long)*cell;
+      *cell = 0;
+      float covered = fabsf(__ll2float_rn(running) * kFixUnit);
+      // An object-level splat is combined without the whole-bin snap (:1137).
+      if (splat) covered = fminf(covered, 1.0f);
+      else if (covered >= 1.0f - 1e-5f) covered = 1.0f;
+      if (covered > 1e-6f) {
+        const float before = st.cov_at(b);
+        float after;
+        if constexpr (WS::kSky) {
+          after = st.independent ? 1.0f - (1.0f - before) * (1.0f - fminf(covered, 1.0f))
+                                 : fmaxf(before, fminf(covered, 1.0f));
+        } else {
+          after = fmaxf(before, fminf(covered, 1.0f));
+        }
+        st.cov_at(b) = after;
+        if (before < 1.0f && after >= 1.0f) st.full++;
       }
-      st.cov_at(b) = after;
-      if (before < 1.0f && after >= 1.0f) st.full++;
     }
+    ws->span_lo[lane] = 68u;
+    ws->span_hi[lane] = 0u;
   }
-  ws->span_lo[lane] = 68u;
-  ws->span_hi[lane] = 0u;
   __syncwarp();
 }
 
 // Stack entry kinds for the walk of both hierarchy levels in one loop.
 constexpr uint32_t kObjNode = 0;   // an object-hierarchy node
-constexpr uint32_t kTriNode = 1;   // a node of the current mesh's triangle hierarchy
-constexpr uint32_t kResolve = 2;   // the current mesh is done: resolve its coverage (index 1: and return to world space)
-constexpr uint32_t kObjRoot = 3;   // instanced scenes: the root of object `index`'s triangle hierarchy
 
 // add_mesh_coverage_if (:713-829) for hierarchy levels 0 and 1: every
 // triangle of mesh m for the lanes with `on`, in leaf-sized groups, then the
@@ -475,7 +543,7 @@ __device__ __forceinline__ void add_mesh_flat(const DevScene& s, LaneState<WS>& 
   }
   if (kCount && on) st.n_tris += range.y;
   for (uint32_t t = range.x; t < range.x + range.y; t += 8)
-    st.queued = cover_leaf(s, st.ws, owners, t, min(8u, range.x + range.y - t), st.queued, lane, st.skip,
+    st.queued = cover_leaf(s.tris, st.ws, owners, t, min(8u, range.x + range.y - t), st.queued, lane, st.skip,
                            st.skips);
   resolve_mesh(s, st, lane);
   if (placed) {
@@ -490,22 +558,403 @@ __device__ __forceinline__ void add_mesh_flat(const DevScene& s, LaneState<WS>& 
   }
 }
 
-// The cone walk (scene_coverage_if, :1160-1227, with add_mesh_coverage_if,
-// :713-829, for each mesh it reaches). Hierarchy level 2 walks both levels in
-// one loop: an object leaf that a lane descends into pushes, for each of its
-// meshes (first mesh on top), a resolve marker under the mesh's triangle
-// hierarchy root, so each mesh is walked and then resolved in the reference's
-// order. Object nodes are visited nearest child first along the bounding
-// cone's axis while some bin is open; triangle-hierarchy nodes right child
-// first (:783-787) with no full check, as in the reference; every popped node
-// a lane needs counts toward its walk cap, though its box was tested when its
+// may_touch_box for the table's cone `owner`. Out of line, for the tests that
+// run seldom: the object walk's, the meshes' roots', the in-order walk's and
+// the tree walk's where box_verdict leaves the question open (about one box in
+// a hundred). The walk is bound by instruction fetch: inline copies at each
+// site cost more than the calls.
+template <class WS>
+static __device__ __noinline__ bool box_in_table(const WS* ws, int owner, f3 lo, f3 hi) {
+  const Cone c = load_cone(ws, owner);
+  return touches_box<WS::kSky>(c, box_test(c), lo, hi, load_horizon(ws, owner));
+}
+template <class WS>
+__device__ __forceinline__ int table_slot(int lane) {
+  return WS::kCones == 32 || lane < WS::kCones ? lane : 0;
+}
+
+// `n` (cone, leaf) pairs from ws->leaves[first], one per lane: each lane
+// takes its cone from the table once and tests its leaf's triangles against
+// it in turn; the survivors join the warp's queue, and every 32 queued pairs
+// are rasterized by the whole warp.
+template <class WS>
+static __device__ __noinline__ uint32_t cull_leaves(const float4* __restrict__ tris, const float4* __restrict__ blas,
+                                                    WS* ws, uint32_t first, uint32_t n, uint32_t queues, int lane,
+                                                    uint32_t skip, bool skips) {
+  uint32_t queued = fast_len(queues), general = general_len(queues);
+  uint32_t t0 = 0, nt = 0;
+  int owner = 0;
+  if ((uint32_t)lane < n) {
+    const uint32_t e = ws->leaves[first + lane];
+    owner = (int)(e >> kQueueOwnerShift);
+    const float4* node = &blas[2 * (size_t)(e & kQueueIndexMask)];
+    t0 = __float_as_uint(__ldg(&node[0].w));
+    nt = __float_as_uint(__ldg(&node[1].w));
+  }
+  const Cone c = load_cone(ws, owner);
+  const f3 horizon = load_horizon(ws, owner);
+  const Corners w = corners_of(c);
+  // The owner's own triangle is not drawn (cover_triangle's cover_skip, :595).
+  [[maybe_unused]] uint32_t own = kNoneU;
+  if constexpr (WS::kBack) {
+    if (skips) own = __shfl_sync(0xffffffffu, skip, owner);
+  }
+  const uint32_t rounds = __reduce_max_sync(0xffffffffu, nt);
+#pragma unroll 1
+  for (uint32_t k = 0; k < rounds; ++k) {
+    bool pass = k < nt && pair_survives<WS::kSky>(tris, c, w, horizon, t0 + k);
+    if constexpr (WS::kBack) {
+      if (t0 + k == own) pass = false;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, pass);
+    if (pass) ws->queue[queued + __popc(m & ((1u << lane) - 1u))] = ((uint32_t)owner << kQueueOwnerShift) | (t0 + k);
+    queued += __popc(m);
+    __syncwarp();
+    if (queued >= 32) {
+      queued -= 32;
+      general = raster_pairs(tris, ws, queued, 32, general, lane);
+    }
+  }
+  return queue_lens(queued, general);
+}
+
+// node_cone_test for the table's cone `owner` and triangle-hierarchy node
+// `node`: drawn into the cone's accumulator where it is splatted.
+template <class WS>
+static __device__ __noinline__ int splat_in_table(WS* ws, int owner, const float4* __restrict__ blas,
+                                                  const float* __restrict__ cov, uint32_t node, float prefilter) {
+  const Cone c = load_cone(ws, owner);
+  const float4 a = __ldg(&blas[2 * (size_t)node]), b = __ldg(&blas[2 * (size_t)node + 1]);
+  LaneAcc<typename WS::Cell, WS::kCones> acc{ws->acc + owner, 68u, 0u, &ws->overflow[0], 1u << owner};
+  const int test = node_cone_test<WS::kSky>(c, load_horizon(ws, owner), acc, cov + kCoverageSamples * (size_t)node,
+                                            node_lo(a), node_lo(b), prefilter);
+  note_span(ws, owner, acc);
+  return test;
+}
+
+// The triangle hierarchy of one mesh in the reference's order (:750-797), a
+// packet of the cones `on`: right child first, each popped node counted
+// against the cone's cap, where the walk stops. The tree walk below leaves to
+// it the cones whose cap ends inside the mesh, and every mesh of a scene whose
+// hierarchies are too deep (DevScene::deep). The stack's entries follow the
+// `base` ones of the walk around it. Returns the queues' lengths, the cone's
+// work, whether its stack overflowed and its visited nodes.
+struct InOrder {
+  uint32_t queued, work, overflowed, nodes;
+};
+template <class WS>
+static __device__ __noinline__ InOrder walk_in_order(const float4* __restrict__ tris, const float4* __restrict__ blas,
+                                                     const float* __restrict__ cov, float prefilter, WS* ws, bool on, uint32_t root, uint32_t work, uint32_t cap,
+                                                     uint32_t queued, int base, int lane, uint32_t skip, bool skips) {
+  const int own = table_slot<WS>(lane);
+  uint32_t overflowed = 0, nodes = 0;
+  WarpStack stk;
+  stk.push(base, root, on, on, lane);
+  int sp = base + 1;
+  bool first = true;  // the root, which the caller counted and tested
+  while (sp > base) {
+    --sp;
+    const uint32_t node = stk.get(sp);
+    const bool mine = stk.need(sp) && (first || work < cap);
+    if (mine && !first) {
+      work++;
+      nodes++;
+    }
+    bool descend = mine && stk.pass(sp);
+    if constexpr (WS::kSplat) {
+      // Every popped node is tested, the root too.
+      if (mine && first) nodes++, work++;
+      if (mine) descend = splat_in_table(ws, own, blas, cov, node, prefilter) == 3;
+    }
+    first = false;
+    const uint32_t owners = __ballot_sync(0xffffffffu, descend);
+    if (!owners) continue;
+    const uint32_t ia = __float_as_uint(__ldg(&blas[2 * (size_t)node].w));
+    const uint32_t ib = __float_as_uint(__ldg(&blas[2 * (size_t)node + 1].w));
+    if (ib > 0) {
+      if (descend) {
+        work += ib;
+        ws->leaves[__popc(owners & ((1u << lane) - 1u))] = ((uint32_t)lane << kQueueOwnerShift) | node;
+      }
+      __syncwarp();
+      queued = cull_leaves(tris, blas, ws, 0, __popc(owners), queued, lane, skip, skips);
+      __syncwarp();
+      continue;
+    }
+    if (sp + 2 > kStack) {
+      if (descend) overflowed = 1;
+      continue;
+    }
+#pragma unroll 1
+    for (int ch = 0; ch < 2; ++ch) {
+      const float4* child = &blas[2 * (size_t)(ia + ch)];
+      const bool p = descend && (WS::kSplat || box_in_table(ws, own, node_lo(__ldg(child)), node_lo(__ldg(child + 1))));
+      stk.push(sp + ch, ia + ch, descend, p, lane);
+    }
+    sp += 2;
+  }
+  return {queued, work, overflowed, nodes};
+}
+
+// The tree walk's steps for prefiltering cones: pairs of a cone and a node,
+// tested when taken (node_cone_test, :519-574). quick_node_test settles most;
+// the others wait until 32 are tested, and drawn, together: in a walk of each
+// node by the whole packet the projections and the hull took every lane's time
+// where a few needed them (prefiltered sky cones over 1 M triangles: 105 ->
+// 34 ms, light cones over 2 M: 33 -> 18.5 ms). A node splatted
+// while its mesh is walked is an integer sum like a triangle's, so its order
+// does not matter either.
+template <bool kCount, class WS>
+__device__ __forceinline__ void walk_splat_pairs(const DevScene& s, LaneState<WS>& st, uint32_t np, int lane,
+                                                 float prefilter) {
+  WS* ws = st.ws;
+  uint32_t nl = 0, ns = 0;
+  const uint32_t below = (1u << lane) - 1u;
+  for (;;) {
+    if (nl >= 32 || (np == 0 && ns == 0 && nl > 0)) {
+      const uint32_t n = min(nl, 32u);
+      nl -= n;
+      st.queued = cull_leaves(s.tris, s.blas, ws, nl, n, st.queued, lane, st.skip, st.skips);
+      continue;
+    }
+    const bool splat = ns >= 32 || (np == 0 && ns > 0);
+    if (!splat && np == 0) break;
+    const int room = WS::kPairs - 2 * kStack - (int)np;
+    const uint32_t n = min(min(splat ? ns : np, 32u), (uint32_t)max(room, 1));
+    uint32_t entry = 0;
+    bool live = false;
+    if ((uint32_t)lane < n) {
+      entry = splat ? ws->splats[ns - n + lane] : ws->pairs[np - n + lane];
+      live = ws->budget[entry >> kQueueOwnerShift] > 0;  // else the cone is walked again in order
+    }
+    if (splat) ns -= n; else np -= n;
+    __syncwarp();
+    const uint32_t owner = entry >> kQueueOwnerShift, node = entry & kQueueIndexMask;
+    int test = 0;
+    uint32_t first = 0, count = 0;
+    if (live) {
+      const float4 a = __ldg(&s.blas[2 * (size_t)node]), b = __ldg(&s.blas[2 * (size_t)node + 1]);
+      first = __float_as_uint(a.w);
+      count = __float_as_uint(b.w);
+      if (splat) {
+        test = splat_in_table(ws, (int)owner, s.blas, s.blas_cov, node, prefilter);
+      } else {
+        const Cone c = load_cone(ws, (int)owner);
+        test = quick_node_test<WS::kSky>(c, box_test(c), node_lo(a), node_lo(b), load_horizon(ws, (int)owner), prefilter);
+        if (kCount) atomicAdd(&ws->visited[owner], 1u);
+      }
+      const int done = (splat ? 0 : 1) + (test == 3 ? (int)count : 0);
+      if (done) atomicSub(&ws->budget[owner], done);
+    }
+    const uint32_t tag = owner << kQueueOwnerShift;
+    const bool leaf = test == 3 && count > 0, inner = test == 3 && count == 0;
+    const uint32_t later = __ballot_sync(0xffffffffu, test == 4), leaves = __ballot_sync(0xffffffffu, leaf),
+                   inners = __ballot_sync(0xffffffffu, inner);
+    if (test == 4) ws->splats[ns + __popc(later & below)] = entry;
+    if (leaf) ws->leaves[nl + __popc(leaves & below)] = tag | node;
+    if (inner) {
+      ws->pairs[np + 2 * __popc(inners & below)] = tag | first;
+      ws->pairs[np + 2 * __popc(inners & below) + 1] = tag | (first + 1u);
+    }
+    ns += __popc(later);
+    nl += __popc(leaves);
+    np += 2 * __popc(inners);
+    __syncwarp();
+  }
+}
+
+// A mesh's triangle hierarchy (add_mesh_coverage_if, :750-797) for every cone
+// that needs it, as pairs of a cone and a node: each step takes up to 32
+// pairs from the warp's stack, one per lane, whichever cones they belong to,
+// and tests both children. Within a mesh the order of the visits does not
+// matter: the accumulated areas are exact integers and no early-out looks at
+// them; only the cap does, and a cone whose work reaches it here is walked
+// again in order (walk_in_order), its accumulator cleared. A packet's cones
+// share few nodes below a mesh's first levels: walked as a union, 9 of 32
+// lanes were active in the box tests and a packet took 252 steps where its
+// cones needed 53 each.
+// `on`: the lane's cone passed the root's box. `base`: the stack entries that
+// the object walk holds. st.queued and st's counters are updated.
+template <bool kCount, class WS>
+__device__ __forceinline__ void walk_tree(const DevScene& s, LaneState<WS>& st, bool on, uint32_t root, int base,
+                                          int lane, [[maybe_unused]] float prefilter) {
+  WS* ws = st.ws;
+  bool in_order = on;
+  if (!s.deep) {
+    const int own = table_slot<WS>(lane);
+    const uint32_t left_over = st.cap - st.cone_work;
+    const int budget = on ? (int)min(left_over, 0x7fffffffu) : 0;
+    const uint32_t owners = __ballot_sync(0xffffffffu, on);
+    const uint32_t at = __popc(owners & ((1u << lane) - 1u));
+    uint32_t np = 0, nl = 0;
+    if constexpr (WS::kSplat) {
+      if (WS::kCones == 32 || lane < WS::kCones) {
+        ws->budget[lane] = budget;
+        ws->visited[lane] = 0u;
+      }
+      if (on) ws->pairs[at] = ((uint32_t)lane << kQueueOwnerShift) | root;
+      np = __popc(owners);
+      __syncwarp();
+      walk_splat_pairs<kCount>(s, st, np, lane, prefilter);
+    } else {
+      const uint32_t ra = __float_as_uint(__ldg(&s.blas[2 * (size_t)root].w));
+      const uint32_t rb = __float_as_uint(__ldg(&s.blas[2 * (size_t)root + 1].w));
+      if (WS::kCones == 32 || lane < WS::kCones) {
+        ws->budget[lane] = budget - (int)(on ? rb : 0u);
+        ws->visited[lane] = 0u;
+      }
+      if (rb == 0) {
+        if (on) ws->pairs[at] = ((uint32_t)lane << kQueueOwnerShift) | ra;
+        np = __popc(owners);
+      } else {
+        if (on) ws->leaves[at] = ((uint32_t)lane << kQueueOwnerShift) | root;
+        nl = __popc(owners);
+      }
+      __syncwarp();
+      for (;;) {
+        if (nl >= 32 || (np == 0 && nl > 0)) {
+          const uint32_t n = min(nl, 32u);
+          nl -= n;
+          st.queued = cull_leaves(s.tris, s.blas, ws, nl, n, st.queued, lane, st.skip, st.skips);
+          continue;
+        }
+        if (np == 0) break;
+        const int room = WS::kPairs - kStack - (int)np;
+        const uint32_t n = min(min(np, 32u), (uint32_t)max(room, 1));
+        np -= n;
+        uint32_t entry = 0;
+        bool live = false;
+        if ((uint32_t)lane < n) {
+          entry = ws->pairs[np + lane];
+          live = ws->budget[entry >> kQueueOwnerShift] > 0;  // else the cone is walked again in order
+        }
+        __syncwarp();
+        const uint32_t owner = entry >> kQueueOwnerShift, left = entry & kQueueIndexMask;
+        bool pl = false, pr = false;
+        uint32_t al = 0, ar = 0, bl = 0, br = 0;
+        if (live) {
+          const float4* rec = s.blas + 2 * (size_t)left;
+          const float4 la = __ldg(rec + 0), lb = __ldg(rec + 1), xa = __ldg(rec + 2), xb = __ldg(rec + 3);
+          const Cone c = load_cone(ws, (int)owner);
+          const f3 horizon = load_horizon(ws, (int)owner);
+          al = __float_as_uint(la.w);
+          bl = __float_as_uint(lb.w);
+          ar = __float_as_uint(xa.w);
+          br = __float_as_uint(xb.w);
+          const BoxTest test = box_test(c);
+  #pragma unroll 1
+          for (int ch = 0; ch < 2; ++ch) {
+            int v = box_verdict<WS::kSky>(c, test, node_lo(ch ? xa : la), node_lo(ch ? xb : lb), horizon);
+            if (v == 2) v = box_in_table(ws, (int)owner, node_lo(ch ? xa : la), node_lo(ch ? xb : lb)) ? 1 : 0;
+            if (ch) pr = v == 1; else pl = v == 1;
+          }
+          // Both children are visited, and a leaf's triangles tested.
+          atomicSub(&ws->budget[owner], (int)(2u + (pl ? bl : 0u) + (pr ? br : 0u)));
+          if (kCount) atomicAdd(&ws->visited[owner], 2u);
+        }
+        const uint32_t tag = owner << kQueueOwnerShift;
+        const uint32_t below = (1u << lane) - 1u;
+        const uint32_t nodes_l = __ballot_sync(0xffffffffu, pl && bl == 0), leaves_l = __ballot_sync(0xffffffffu, pl && bl);
+        const uint32_t nodes_r = __ballot_sync(0xffffffffu, pr && br == 0), leaves_r = __ballot_sync(0xffffffffu, pr && br);
+        if (pl) {
+          if (bl) ws->leaves[nl + __popc(leaves_l & below)] = tag | left;
+          else ws->pairs[np + __popc(nodes_l & below)] = tag | al;
+        }
+        np += __popc(nodes_l);
+        nl += __popc(leaves_l);
+        if (pr) {
+          if (br) ws->leaves[nl + __popc(leaves_r & below)] = tag | (left + 1u);
+          else ws->pairs[np + __popc(nodes_r & below)] = tag | ar;
+        }
+        np += __popc(nodes_r);
+        nl += __popc(leaves_r);
+        __syncwarp();
+      }
+    }
+    const int after = ws->budget[own];
+    in_order = on && after <= 0;
+    if (on && !in_order) {
+      const uint32_t done = (uint32_t)(budget - after);
+      st.cone_work += done;
+      if (kCount) {
+        st.n_blas += ws->visited[own];
+        st.n_tris += done - ws->visited[own];
+      }
+    }
+    const uint32_t again = __ballot_sync(0xffffffffu, in_order);
+    if (again) {
+      // Their areas so far are dropped.
+      drain_queues(s.tris, ws, st.queued, lane);
+      if (in_order) {
+#pragma unroll 1
+        for (int b = 0; b < kBins; ++b) ws->acc[WS::kCones * b + lane] = 0;
+        ws->span_lo[lane] = 68u;
+        ws->span_hi[lane] = 0u;
+      }
+      if (lane == 0) ws->overflow[0] &= ~again;
+      __syncwarp();
+    }
+  }
+  if (__any_sync(0xffffffffu, in_order)) {
+    const InOrder r = walk_in_order(s.tris, s.blas, s.blas_cov, prefilter, ws, in_order, root, st.cone_work, st.cap, st.queued, base, lane,
+                                    st.skip, st.skips);
+    st.queued = r.queued;
+    if (r.overflowed) st.status |= 2u;
+    if (kCount) {
+      st.n_blas += r.nodes;
+      st.n_tris += r.work - st.cone_work - r.nodes;
+    }
+    st.cone_work = r.work;
+  }
+}
+
+// One mesh that the lanes with `descend` reach (add_mesh_coverage_if,
+// :713-829): its root's box in the mesh's own space, its triangle hierarchy,
+// and the resolve of its coverage into the mask.
+template <bool kCount, bool kInst, class WS>
+__device__ __forceinline__ void add_mesh_tree(const DevScene& s, LaneState<WS>& st, bool descend, uint4 range,
+                                              int base, int lane) {
+  const float4 ma = __ldg(&s.blas[2 * (size_t)range.z + 0]);
+  const float4 mb = __ldg(&s.blas[2 * (size_t)range.z + 1]);
+  const bool mine = descend && st.cone_work < st.cap;
+  if (mine) {
+    st.cone_work++;
+    if (kCount) st.n_blas++;
+  }
+  const bool placed = kInst && range.w != kNoneU;
+  if (placed) {
+    // A placed object: the cone in its space (cone_to_object, :623-638), the
+    // horizon turned with it (:634).
+    const float4* X = s.xforms + 4 * (size_t)range.w;
+    store_cone(st.ws, cone_to_object(world_cone(st), X), lane);
+    if constexpr (WS::kSky) store_horizon(st.ws, rotate_to_object(st.horizon, X), lane);
+    enter_object(st.ws, X, lane);
+    __syncwarp();
+  }
+  const bool on = mine && box_in_table(st.ws, table_slot<WS>(lane), node_lo(ma), node_lo(mb));
+  if (__any_sync(0xffffffffu, on)) {
+    walk_tree<kCount>(s, st, on, range.z, base, lane, 0.0f);
+    resolve_mesh(s, st, lane);
+  }
+  if (placed) {  // back to world space
+    store_cone(st.ws, world_cone(st), lane);
+    store_horizon(st.ws, st.horizon, lane);
+    leave_object(st.ws, lane);
+    __syncwarp();
+  }
+}
+
+// The cone walk (scene_coverage_if, :1160-1227). The packet walks the object
+// hierarchy, nearest child first along the bounding cone's axis while some
+// bin is open, and each mesh of a leaf that a lane descends into is walked
+// and resolved in the reference's order (add_mesh_tree). Every popped node a
+// lane needs counts toward its walk cap, though its box was tested when its
 // parent was visited. Levels 0 and 1 keep the reference's loops over meshes
 // and triangles; they are compiled only into the kernels of kFlat, which
 // launches at those levels take, so the level-2 walk's code stays small.
 template <bool kCount, bool kInst, bool kFlat, class WS>
 __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy, LaneState<WS>& st, bool traced,
                                            int lane) {
-  const Cone& c = st.cone;
   if constexpr (kFlat) {
     if (hierarchy == 0) {
       for (uint32_t m = 0; m < s.nmeshes; ++m)
@@ -513,64 +962,26 @@ __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy
       return;
     }
   }
+  const int own = table_slot<WS>(lane);
   WarpStack stk;
   const float4 ra = __ldg(&s.nodes[0]);
   const float4 rb = __ldg(&s.nodes[1]);
-  const bool root_pass = traced && may_touch_box<WS::kSky, false>(c, node_lo(ra), node_lo(rb), st.horizon);
+  const bool root_pass = traced && box_in_table(st.ws, own, node_lo(ra), node_lo(rb));
   stk.push(0, node_ref(ra, rb, kObjNode), traced, root_pass, lane);
   int sp = 1;
   while (sp > 0) {
     --sp;
-    uint32_t ref = stk.get(sp);
-    uint32_t kind = ref_kind(ref);
-    if (kind == kResolve) {
-      resolve_mesh(s, st, lane);
-      if (kInst && ref_index(ref) == 1) {  // back to world space
-        st.cone = st.world;
-        store_cone(st.ws, st.cone, lane);
-        leave_object(st.ws, lane);
-        if constexpr (WS::kSky) {
-          st.horizon = st.world_horizon;
-          store_horizon(st.ws, st.horizon, lane);
-        }
-        __syncwarp();
-      }
-      continue;
-    }
-    if (kInst && kind == kObjRoot) {
-      // Entering a placed object: the cone in its space (cone_to_object,
-      // :623-638), then its triangle hierarchy's root.
-      const uint4 range = __ldg(&s.meshes[ref_index(ref)]);
-      st.cone = cone_to_object(st.world, s.xforms + 4 * (size_t)range.w);
-      store_cone(st.ws, st.cone, lane);
-      enter_object(st.ws, s.xforms + 4 * (size_t)range.w, lane);
-      if constexpr (WS::kSky) {
-        // The horizon turns with the cone (:634).
-        st.horizon = rotate_to_object(st.world_horizon, s.xforms + 4 * (size_t)range.w);
-        store_horizon(st.ws, st.horizon, lane);
-      }
-      __syncwarp();
-      ref = node_ref(__ldg(&s.blas[2 * (size_t)range.z + 0]), __ldg(&s.blas[2 * (size_t)range.z + 1]), kTriNode);
-      kind = kTriNode;
-    }
-    const bool is_obj = kind == kObjNode;
-    const bool mine = stk.need(sp) && st.cone_work < st.cap && (!is_obj || st.full < (uint32_t)kBins);
-    if (mine) st.cone_work++;
-    if (kCount && mine) {
-      if (is_obj) st.n_obj++; else st.n_blas++;
+    const uint32_t ref = stk.get(sp);
+    const bool mine = stk.need(sp) && st.cone_work < st.cap && st.full < (uint32_t)kBins;
+    if (mine) {
+      st.cone_work++;
+      if (kCount) st.n_obj++;
     }
     const bool descend = mine && stk.pass(sp);
     const uint32_t owners = __ballot_sync(0xffffffffu, descend);
     if (!owners) continue;
     const uint32_t ia = ref_index(ref), ib = ref_count(ref);
-    if (ib > 0 && !is_obj) {
-      // A triangle-hierarchy leaf: its triangles against every descending cone.
-      if (descend) {
-        st.cone_work += ib;
-        if (kCount) st.n_tris += ib;
-      }
-      st.queued = cover_leaf(s, st.ws, owners, ia, ib, st.queued, lane, st.skip, st.skips);
-    } else if (ib > 0) {
+    if (ib > 0) {
       // An object leaf: its meshes.
       if constexpr (kFlat) {
         if (hierarchy == 1) {
@@ -579,51 +990,41 @@ __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy
           continue;
         }
       }
-      for (int k = (int)(ia + ib) - 1; k >= (int)ia; --k) {
+      // The stack holds the leaf's later meshes, two entries each.
+      int later = sp;
+      for (uint32_t k = ia; k < ia + ib; ++k)
+        if (__ldg(&s.meshes[__ldg(&s.items[k])].z) != kNoneU) later += 2;
+#pragma unroll 1
+      for (uint32_t k = ia; k < ia + ib; ++k) {
         const uint4 range = __ldg(&s.meshes[__ldg(&s.items[k])]);
         if (range.z == kNoneU) continue;  // no triangles: nothing to draw or resolve
-        if (sp + 2 > kStack) {
+        later -= 2;
+        if (later + 2 > kStack) {
           if (descend) st.status |= 2u;
           continue;
         }
-        const float4 ma = __ldg(&s.blas[2 * (size_t)range.z + 0]);
-        const float4 mb = __ldg(&s.blas[2 * (size_t)range.z + 1]);
-        const uint32_t m = __ldg(&s.items[k]);
-        if (kInst && range.w != kNoneU) {
-          // A placed object: its root's box in its own space; the entry names
-          // the object, whose cone is set up when the entry is popped.
-          const Cone oc = cone_to_object(st.world, s.xforms + 4 * (size_t)range.w);
-          f3 oh = st.horizon;
-          if constexpr (WS::kSky) oh = rotate_to_object(st.world_horizon, s.xforms + 4 * (size_t)range.w);
-          const bool mesh_pass = descend && may_touch_box<WS::kSky>(oc, node_lo(ma), node_lo(mb), oh);
-          stk.push(sp, (kResolve << kRefKindShift) | 1u, false, false, lane);
-          stk.push(sp + 1, (kObjRoot << kRefKindShift) | m, descend, mesh_pass, lane);
-        } else {
-          const bool mesh_pass = descend && may_touch_box<WS::kSky, false>(c, node_lo(ma), node_lo(mb), st.horizon);
-          stk.push(sp, kResolve << kRefKindShift, false, false, lane);
-          stk.push(sp + 1, node_ref(ma, mb, kTriNode), descend, mesh_pass, lane);
-        }
-        sp += 2;
+        add_mesh_tree<kCount, kInst>(s, st, descend, range, later + 1, lane);
       }
     } else {
       // An interior node: both children's boxes tested now.
-      const float4* base = (is_obj ? s.nodes : s.blas) + 2 * (size_t)ia;
+      const float4* base = s.nodes + 2 * (size_t)ia;
       const float4 la = __ldg(base + 0), lb = __ldg(base + 1), xa = __ldg(base + 2), xb = __ldg(base + 3);
       bool pl = false, pr = false;
       if (descend) {
 #pragma unroll 1
         for (int ch = 0; ch < 2; ++ch) {
-          const bool t = may_touch_box<WS::kSky>(c, node_lo(ch ? xa : la), node_lo(ch ? xb : lb), st.horizon);
+          const bool t = box_in_table(st.ws, own, node_lo(ch ? xa : la), node_lo(ch ? xb : lb));
           if (ch) pr = t; else pl = t;
         }
       }
-      bool swap = false;  // left child popped first (object level: when it is the nearer)
+      bool swap = false;  // left child popped first (unless the right is the nearer)
       // Nearest child first where meshes combine by the maximum; sky cones
       // combining as independent occluders keep the left child first, as
       // their products would round differently in another order (:1188-1207).
-      bool nearest = is_obj;
-      if constexpr (WS::kSky) nearest = nearest && !st.independent;
+      bool nearest = true;
+      if constexpr (WS::kSky) nearest = !st.independent;
       if (nearest) {
+        const Cone c = load_cone(st.ws, own);
         const float da = dot(c.baxis, (node_lo(la) + node_lo(lb)) * 0.5f - c.apex);
         const float db = dot(c.baxis, (node_lo(xa) + node_lo(xb)) * 0.5f - c.apex);
         const bool pref = db < da;  // this lane's own order: right child nearer
@@ -632,14 +1033,12 @@ __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy
         // could matter).
         swap = 2u * __popc(__ballot_sync(0xffffffffu, descend && pref)) > __popc(owners);
         if (descend && pref != swap) st.status |= 4u;
-      } else if (!is_obj) {
-        swap = true;  // triangle hierarchies pop the right child first (:783-787)
       }
       if (sp + 2 > kStack) {
         if (descend) st.status |= 2u;
         continue;
       }
-      const uint32_t rl = node_ref(la, lb, kind), rr = node_ref(xa, xb, kind);
+      const uint32_t rl = node_ref(la, lb, kObjNode), rr = node_ref(xa, xb, kObjNode);
       // The child popped second below the one popped first.
       stk.push(sp, swap ? rl : rr, descend, swap ? pl : pr, lane);
       stk.push(sp + 1, swap ? rr : rl, descend, swap ? pr : pl, lane);
@@ -650,126 +1049,85 @@ __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy
 
 // The walk of prefiltering cones (hierarchy level 2): scene_coverage_if
 // (:1160-1227) with splat_object_node (:1096-1150) and add_mesh_coverage_if
-// (:750-790) with node_cone_test (:519-574). Each entry is a node index, and
-// a node is tested when popped, as the reference tests it: a node small in
-// the cone is splatted instead of descended into (a triangle-hierarchy node
-// into its mesh's accumulator, an object node into the mask as one more
-// mesh), and the walk cap counts the popped nodes a lane needs.
-constexpr uint32_t kSplatIndexMask = (1u << kRefKindShift) - 1u;
-
+// (:750-790) with node_cone_test (:519-574). An object node is tested when
+// popped, as the reference tests it: one small in the cone is splatted into
+// the mask as one more mesh instead of descended into. A leaf's meshes are
+// walked as the exact cones' are (walk_tree), their nodes tested when taken.
 template <bool kCount, bool kInst, class WS>
 __device__ __forceinline__ void scene_walk_splat(const DevScene& s, float prefilter, LaneState<WS>& st, bool traced,
                                                  int lane) {
   WS* ws = st.ws;
   WarpStack stk;
-  stk.push(0, (kObjNode << kRefKindShift) | 0u, traced, true, lane);
+  stk.push(0, 0u, traced, true, lane);
   int sp = 1;
   while (sp > 0) {
     --sp;
-    const uint32_t entry = stk.get(sp);
-    uint32_t kind = entry >> kRefKindShift;
-    uint32_t idx = entry & kSplatIndexMask;
-    if (kind == kResolve) {
-      resolve_mesh(s, st, lane);
-      if (kInst && idx == 1) {  // back to world space
-        st.cone = st.world;
-        store_cone(ws, st.cone, lane);
-        leave_object(ws, lane);
-        if constexpr (WS::kSky) {
-          st.horizon = st.world_horizon;
-          store_horizon(ws, st.horizon, lane);
-        }
-        __syncwarp();
-      }
-      continue;
-    }
-    if (kInst && kind == kObjRoot) {
-      // Entering a placed object: the cone (and horizon) in its space, then
-      // its triangle hierarchy's root, tested as any popped node.
-      const uint4 range = __ldg(&s.meshes[idx]);
-      st.cone = cone_to_object(st.world, s.xforms + 4 * (size_t)range.w);
-      store_cone(ws, st.cone, lane);
-      enter_object(ws, s.xforms + 4 * (size_t)range.w, lane);
-      if constexpr (WS::kSky) {
-        st.horizon = rotate_to_object(st.world_horizon, s.xforms + 4 * (size_t)range.w);
-        store_horizon(ws, st.horizon, lane);
-      }
-      __syncwarp();
-      kind = kTriNode;
-      idx = range.z;
-    }
-    const bool is_obj = kind == kObjNode;
-    const bool mine = stk.need(sp) && st.cone_work < st.cap && (!is_obj || st.full < (uint32_t)kBins);
-    if (mine) st.cone_work++;
-    if (kCount && mine) {
-      if (is_obj) st.n_obj++; else st.n_blas++;
+    const uint32_t idx = stk.get(sp);
+    const bool mine = stk.need(sp) && st.cone_work < st.cap && st.full < (uint32_t)kBins;
+    if (mine) {
+      st.cone_work++;
+      if (kCount) st.n_obj++;
     }
     if (!__any_sync(0xffffffffu, mine)) continue;
-    const float4* rec = (is_obj ? s.nodes : s.blas) + 2 * (size_t)idx;
-    const float4 ra = __ldg(rec), rb = __ldg(rec + 1);
+    const float4 ra = __ldg(&s.nodes[2 * (size_t)idx]), rb = __ldg(&s.nodes[2 * (size_t)idx + 1]);
     const f3 lo = node_lo(ra), hi = node_lo(rb);
-    const uint32_t ref = node_ref(ra, rb, kind);
-    const uint32_t ia = ref_index(ref), ib = ref_count(ref);
-    bool descend = false;
-    if (is_obj) {
-      bool splatted = false;
-      if (mine && may_touch_box<WS::kSky>(st.cone, lo, hi, st.horizon)) {
-        const float* cov = s.obj_cov ? s.obj_cov + kCoverageSamples * (size_t)idx : nullptr;
-        if (cov && __ldg(&cov[13]) == 0.0f) {
-          LaneAcc<typename WS::Cell> acc{ws->acc + lane, 68u, 0u, &ws->overflow[0], 1u << lane};
-          splatted = splat_object_node(st.cone, acc, cov, lo, hi, prefilter);
-          if (acc.span_lo < acc.span_hi) {
-            ws->span_lo[lane] = min(ws->span_lo[lane], acc.span_lo);
-            ws->span_hi[lane] = max(ws->span_hi[lane], acc.span_hi);
-          }
-        }
-        descend = !splatted;
+    const uint32_t ia = __float_as_uint(ra.w), ib = __float_as_uint(rb.w);
+    bool splatted = false, descend = false;
+    if (mine && box_in_table(ws, table_slot<WS>(lane), lo, hi)) {
+      const float* cov = s.obj_cov ? s.obj_cov + kCoverageSamples * (size_t)idx : nullptr;
+      if (cov && __ldg(&cov[13]) == 0.0f) {
+        LaneAcc<typename WS::Cell, WS::kCones> acc{ws->acc + lane, 68u, 0u, &ws->overflow[0], 1u << lane};
+        splatted = splat_object_node(st.cone, acc, cov, lo, hi, prefilter);
+        note_span(ws, lane, acc);
       }
-      // Splats are combined into the mask at once, as one more mesh each.
-      if (__any_sync(0xffffffffu, splatted)) resolve_mesh(s, st, lane, true);
-    } else if (mine) {
-      LaneAcc<typename WS::Cell> acc{ws->acc + lane, 68u, 0u, &ws->overflow[0], 1u << lane};
-      const int test = node_cone_test<WS::kSky>(st.cone, st.horizon, acc, s.blas_cov + kCoverageSamples * (size_t)idx,
-                                                lo, hi, prefilter);
-      if (acc.span_lo < acc.span_hi) {
-        ws->span_lo[lane] = min(ws->span_lo[lane], acc.span_lo);
-        ws->span_hi[lane] = max(ws->span_hi[lane], acc.span_hi);
-      }
-      descend = test == 3;
+      descend = !splatted;
     }
+    // Splats are combined into the mask at once, as one more mesh each.
+    if (__any_sync(0xffffffffu, splatted)) resolve_mesh(s, st, lane, true);
     const uint32_t owners = __ballot_sync(0xffffffffu, descend);
     if (!owners) continue;
-    if (is_obj && ib > 0) {
-      // An object leaf: its meshes, first on top, each under its resolve marker.
-      for (int k = (int)(ia + ib) - 1; k >= (int)ia; --k) {
-        const uint32_t m = __ldg(&s.items[k]);
-        const uint4 range = __ldg(&s.meshes[m]);
+    if (ib > 0) {
+      // An object leaf: its meshes; the stack holds the later ones, two
+      // entries each.
+      int later = sp;
+      for (uint32_t k = ia; k < ia + ib; ++k)
+        if (__ldg(&s.meshes[__ldg(&s.items[k])].z) != kNoneU) later += 2;
+#pragma unroll 1
+      for (uint32_t k = ia; k < ia + ib; ++k) {
+        const uint4 range = __ldg(&s.meshes[__ldg(&s.items[k])]);
         if (range.z == kNoneU) continue;  // no triangles: nothing to draw or resolve
-        if (sp + 2 > kStack) {
+        later -= 2;
+        if (later + 2 > kStack) {
           if (descend) st.status |= 2u;
           continue;
         }
+        const bool on = descend && st.cone_work < st.cap;
+        if (!__any_sync(0xffffffffu, on)) continue;
         const bool placed = kInst && range.w != kNoneU;
-        stk.push(sp, (kResolve << kRefKindShift) | (placed ? 1u : 0u), false, false, lane);
-        stk.push(sp + 1, placed ? ((kObjRoot << kRefKindShift) | m) : ((kTriNode << kRefKindShift) | range.z), descend,
-                 true, lane);
-        sp += 2;
+        const float4* X = s.xforms + 4 * (size_t)range.w;
+        if (placed) {
+          // The cone (and horizon) in the object's space.
+          store_cone(ws, cone_to_object(st.cone, X), lane);
+          if constexpr (WS::kSky) store_horizon(ws, rotate_to_object(st.horizon, X), lane);
+          enter_object(ws, X, lane);
+          __syncwarp();
+        }
+        walk_tree<kCount>(s, st, on, range.z, later + 1, lane, prefilter);
+        resolve_mesh(s, st, lane);
+        if (placed) {  // back to world space
+          store_cone(ws, st.cone, lane);
+          store_horizon(ws, st.horizon, lane);
+          leave_object(ws, lane);
+          __syncwarp();
+        }
       }
-    } else if (!is_obj && ib > 0) {
-      // A triangle-hierarchy leaf: its triangles against every descending cone.
-      if (descend) {
-        st.cone_work += ib;
-        if (kCount) st.n_tris += ib;
-      }
-      st.queued = cover_leaf(s, ws, owners, ia, ib, st.queued, lane, st.skip, st.skips);
     } else {
       if (sp + 2 > kStack) {
         if (descend) st.status |= 2u;
         continue;
       }
-      bool swap = !is_obj;  // triangle hierarchies pop the right child first (:783-787)
-      bool nearest = is_obj;
-      if constexpr (WS::kSky) nearest = nearest && !st.independent;
+      bool swap = false, nearest = true;
+      if constexpr (WS::kSky) nearest = !st.independent;
       if (nearest) {
         const float4* base = s.nodes + 2 * (size_t)ia;
         const float4 la = __ldg(base + 0), lb = __ldg(base + 1), xa = __ldg(base + 2), xb = __ldg(base + 3);
@@ -779,9 +1137,8 @@ __device__ __forceinline__ void scene_walk_splat(const DevScene& s, float prefil
         swap = 2u * __popc(__ballot_sync(0xffffffffu, descend && pref)) > __popc(owners);  // the majority's order
         if (descend && pref != swap) st.status |= 4u;
       }
-      const uint32_t l = (kind << kRefKindShift) | ia, r = (kind << kRefKindShift) | (ia + 1u);
-      stk.push(sp, swap ? l : r, descend, true, lane);
-      stk.push(sp + 1, swap ? r : l, descend, true, lane);
+      stk.push(sp, swap ? ia : ia + 1u, descend, true, lane);
+      stk.push(sp + 1, swap ? ia + 1u : ia, descend, true, lane);
       sp += 2;
     }
   }
@@ -959,11 +1316,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, resident_blocks<kWide, kS
   // a tenth of the kernel's code, which competes for the instruction caches
   // with the walk.
 #pragma unroll 1
-  for (int k = 0; k < kBins; ++k) ws->acc[32 * k + lane] = 0;
+  for (int k = lane; k < kBins * WS::kCones; k += 32) ws->acc[k] = 0;
   if (lane == 0) ws->overflow[0] = 0u;
   leave_object(ws, lane);  // the world's weight until a placed object is entered
-  ws->span_lo[lane] = 68u;
-  ws->span_hi[lane] = 0u;
+  if (lane < WS::kCones) {
+    ws->span_lo[lane] = 68u;
+    ws->span_hi[lane] = 0u;
+  }
 
   // The split path (exact light cones): the walk takes each slot's cone from
   // its record, set up by cone_setup_kernel, and leaves its mask to
@@ -1084,19 +1443,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, resident_blocks<kWide, kS
     LightConeInfo info{true, false, false};
     bool traced;
     if constexpr (kSplit) {
-      // The cone as cone_setup_kernel set it up.
-      st.cone.apex = mk(rec.a.x, rec.a.y, rec.a.z);
-      st.cone.far_offset = rec.a.w;
-      st.cone.right = mk(rec.b.x, rec.b.y, rec.b.z);
-      st.cone.u0 = rec.b.w;
-      st.cone.up = mk(rec.c.x, rec.c.y, rec.c.z);
-      st.cone.v0 = rec.c.w;
-      st.cone.fwd = mk(rec.d.x, rec.d.y, rec.d.z);
-      st.cone.u1 = rec.d.w;
-      st.cone.baxis = mk(rec.e.x, rec.e.y, rec.e.z);
-      st.cone.v1 = rec.e.w;
-      st.cone.bcos = rec.f.x;
-      st.cone.bsin = rec.f.y;
+      st.cone = record_cone(rec);
+      st.rec = &records[slot_local];
       const uint32_t flags = __float_as_uint(rec.f.w);
       traced = valid && (flags & 1u);
       st.skip = valid ? (flags >> 4) - 1u : kNoneU;
@@ -1166,6 +1514,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, resident_blocks<kWide, kS
     if constexpr (WS::kSky) {
       // sky_face_light (:1489-1498): the face's window clipped to the
       // horizon, less its covered bins' clipped weights.
+      if constexpr (!kSplat && !kInst) st.cone = load_cone(ws, table_slot<WS>(lane));
       if (traced) {
         float blocked = 0.0f;
 #pragma unroll 1

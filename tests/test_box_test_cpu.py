@@ -1,0 +1,124 @@
+"""The short box test against the exact one, on the host.
+
+box_test.cuh's box_verdict must never contradict may_touch_box: it answers
+only where f32 rounding cannot change the answer, and leaves the rest to it.
+The header is compiled with the host compiler (no contraction, as the walk's
+units) over random cones and boxes of every size, boxes with a corner on a
+window plane, flat boxes, sky faces, and values that are not finite.
+"""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+HARNESS = r"""
+#include <cmath>
+#include <cstdio>
+#include <random>
+#define __device__
+#define __forceinline__ inline
+#define __fmaf_rn fmaf
+namespace cc {
+struct f3 { float x, y, z; };
+static f3 mk(float x, float y, float z) { return {x, y, z}; }
+static f3 operator+(f3 a, f3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
+static f3 operator-(f3 a, f3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+static f3 operator-(f3 a) { return {-a.x, -a.y, -a.z}; }
+static f3 operator*(f3 a, float s) { return {a.x * s, a.y * s, a.z * s}; }
+static float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+static f3 cross(f3 a, f3 b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
+static float len(f3 a) { return sqrtf(dot(a, a)); }
+static f3 normalize(f3 a) { const float l = len(a); return {a.x / l, a.y / l, a.z / l}; }
+constexpr float kNear = 1e-4f;
+struct Cone { f3 apex, right, up, fwd; float u0, v0, u1, v1, far_offset; f3 baxis; float bcos, bsin; };
+static f3 direction(const Cone& c, float s, float t) {
+  return c.fwd + c.right * (c.u0 + s * (c.u1 - c.u0)) + c.up * (c.v0 + t * (c.v1 - c.v0));
+}
+static f3 to_local(const Cone& c, f3 p) { const f3 d = p - c.apex; return {dot(c.right, d), dot(c.up, d), dot(c.fwd, d)}; }
+static float min_nan(float a, float b) { return std::isnan(a) || std::isnan(b) ? NAN : fminf(a, b); }
+static float rsqrt_approx(float x) { return (float)(1.0 / std::sqrt((double)x)) * (1.0f + 2e-7f); }
+#include "box_test.cuh"
+}  // namespace cc
+using namespace cc;
+int main(int, char** argv) {
+  std::mt19937_64 g(atoi(argv[1]));
+  auto u = [&] { return (double)(g() >> 11) / 9007199254740992.0; };
+  auto U = [&](double a, double b) { return (float)(a + (b - a) * u()); };
+  auto L = [&](double a, double b) { return (float)std::exp(std::log(a) + (std::log(b) - std::log(a)) * u()); };
+  long asked = 0, open = 0, wrong = 0;
+  for (long it = 0; it < 60000; ++it) {
+    const float world = L(0.5, 3000);
+    Cone c{};
+    c.apex = mk(U(-world, world), U(0, world * 0.1), U(-world, world));
+    const f3 f = normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)));
+    c.fwd = f;
+    c.right = normalize(cross(std::fabs(f.x) > 0.9f ? mk(0, 1, 0) : mk(1, 0, 0), f));
+    c.up = cross(f, c.right);
+    const bool sky = it % 11 == 0;
+    if (it % 7 == 0 || sky) {
+      c.fwd = mk(0, it % 2 ? 1.f : -1.f, 0);
+      c.right = mk(0, 0, 1);
+      c.up = cross(c.fwd, c.right);
+    }
+    const float ext = L(0.003, 12);
+    c.u0 = U(-3, 3);
+    c.v0 = U(-3, 3);
+    c.u1 = c.u0 + ext;
+    c.v1 = c.v0 + ext * U(0.3, 1);
+    if (sky) { c.u0 = c.v0 = -1; c.u1 = c.v1 = 1; }
+    const float dist = L(0.01, world * 1.5);
+    c.far_offset = dot(c.fwd, c.apex) + (sky ? 1e7f : dist * (1 - 1e-5f));
+    c.baxis = normalize(direction(c, 0.5f, 0.5f));
+    float ch = 1;
+    for (int k = 0; k < 4; ++k) ch = fminf(ch, dot(c.baxis, normalize(direction(c, float(k & 1), float(k >> 1)))));
+    c.bcos = fminf(fmaxf(ch - 1e-5f, -1.f), 1.f);
+    c.bsin = sqrtf(fmaxf(1.f - c.bcos * c.bcos, 0.f));
+    const f3 hz = normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)));
+    if (it % 5003 == 1) c.right.x = NAN;
+    if (it % 5003 == 2) c.baxis.y = NAN;
+    if (it % 5003 == 3) c.apex.z = INFINITY;
+    const BoxTest t = box_test(c);
+    for (int k = 0; k < 24; ++k) {
+      const float size = L(0.001, world);
+      f3 e = mk(L(0.01, 1) * size, L(0.01, 1) * size, L(0.01, 1) * size);
+      if (k % 5 == 0) e.y = 0;
+      const float z = L(1e-4, dist * 2), uu = c.u0 + (c.u1 - c.u0) * U(-0.3, 1.3), vv = c.v0 + (c.v1 - c.v0) * U(-0.3, 1.3);
+      f3 at = c.apex + (c.fwd + c.right * uu + c.up * vv) * z;
+      if (k % 4 == 0) at = mk(U(-world, world), U(-world, world), U(-world, world));
+      f3 lo = at - e * 0.5f, hi = at + e * 0.5f;
+      if (k % 6 == 1) {  // a corner on the window's first side
+        const f3 p = c.apex + (c.fwd + c.right * c.u0 + c.up * vv) * z;
+        const f3 q = mk(c.right.x > 0 ? p.x - e.x : p.x + e.x, c.right.y > 0 ? p.y - e.y : p.y + e.y,
+                        c.right.z > 0 ? p.z - e.z : p.z + e.z);
+        lo = mk(fminf(p.x, q.x), fminf(p.y, q.y), fminf(p.z, q.z));
+        hi = mk(fmaxf(p.x, q.x), fmaxf(p.y, q.y), fmaxf(p.z, q.z));
+      }
+      if (it % 5003 == 4) hi.x = INFINITY;
+      for (int h = 0; h < 2; ++h) {
+        const bool exact = h ? may_touch_box<true>(c, lo, hi, hz) : may_touch_box<false>(c, lo, hi, hz);
+        const int v = h ? box_verdict<true>(c, t, lo, hi, hz) : box_verdict<false>(c, t, lo, hi, hz);
+        ++asked;
+        if (v == 2) ++open;
+        else if ((v == 1) != exact) ++wrong;
+      }
+    }
+  }
+  std::printf("%ld %ld %ld\n", asked, open, wrong);
+}
+"""
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_box_verdict_never_contradicts_the_exact_test(tmp_path, seed):
+    src = tmp_path / "box.cpp"
+    src.write_text(HARNESS)
+    exe = tmp_path / "box"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-Wno-unknown-pragmas", "-I",
+                    str(ROOT / "continuum_b200" / "csrc"), "-o", str(exe), str(src)], check=True)
+    asked, left, wrong = map(int, subprocess.run([str(exe), str(seed)], check=True, capture_output=True,
+                                                 text=True).stdout.split())
+    assert wrong == 0
+    # A sixth of the boxes are put on a plane; most others are decided.
+    assert left < 0.25 * asked
