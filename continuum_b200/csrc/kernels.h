@@ -236,6 +236,7 @@ cudaError_t upload_disk_table(const float* table64);
 // The prefiltering unit's copy of the table, and its plain passes (packet
 // pass with 32-bit cells, or solo pass with 64-bit ones when `wide`).
 cudaError_t upload_disk_table_splat(const float* table64);
+cudaError_t make_sky_table_splat();  // its copy of the sky faces' directions (default stream)
 cudaError_t launch_splat_pass(bool wide, bool count, bool inst, bool sky, const DevScene& s, const DevQuery& q,
                               const DevOut& o, const uint32_t* list, const uint32_t* list_count, uint32_t pw,
                               uint32_t blocks, cudaStream_t stream);

@@ -36,8 +36,12 @@ namespace cc {
 cudaError_t upload_disk_table(const float* table64) {
   cudaError_t e = cudaMemcpyToSymbol(c_disk, table64, kBins * sizeof(float));
   if (e == cudaSuccess) e = upload_disk_table_split(table64);  // the integrating unit's copy
+  if (e == cudaSuccess) e = upload_disk_table_splat(table64);  // the prefiltering unit's copy
   if (e != cudaSuccess) return e;
-  return upload_disk_table_splat(table64);  // the prefiltering unit's copy
+  sky_table_kernel<<<6, 160>>>();
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = make_sky_table_splat();
+  return e == cudaSuccess ? cudaDeviceSynchronize() : e;
 }
 
 // The exact cones' plain pass (packet or solo) of the variant the flags pick;

@@ -1218,6 +1218,68 @@ static __device__ __noinline__ float warp_blocked(const Cone& mine, f3 my_normal
   return sum;
 }
 
+// The sky faces in world axes: every receiver's face has the same frame and
+// window, so the directions of its 81 bin corners and, of its 144 bin edges
+// (72 along rows, then 72 along columns), the angle and the unit normal of the
+// plane through the apex (lambert_edge_unit's parts that do not depend on the
+// receiver) are the same: made once per device by sky_table_kernel.
+struct SkyFaces {
+  float4 corner[6][81];
+  float4 edge[6][144];  // unit normal, angle
+};
+static __device__ SkyFaces g_sky_faces;
+
+// Static, like the table: each unit fills its own.
+[[maybe_unused]] static __global__ void sky_table_kernel() {
+  const uint32_t f = blockIdx.x;
+  Cone c{};
+  sky_face(f, mk(0.f, 0.f, 0.f), mk(0.f, 1.f, 0.f), c);
+  const float g = float(kGrid);
+  for (int p = threadIdx.x; p < 81; p += blockDim.x) {
+    const f3 d = direction(c, float(p % 9) / g, float(p / 9) / g);
+    g_sky_faces.corner[f][p] = make_float4(d.x, d.y, d.z, 0.f);
+  }
+  for (int e = threadIdx.x; e < 144; e += blockDim.x) {
+    const int a = e < 72 ? (e / 8) * 9 + e % 8 : e - 72, b = e < 72 ? a + 1 : a + 9;
+    const f3 u = normalize(direction(c, float(a % 9) / g, float(a / 9) / g));
+    const f3 v = normalize(direction(c, float(b % 9) / g, float(b / 9) / g));
+    const f3 n = cross(u, v);
+    const float l = len(n);
+    const f3 unit = l > 1e-12f ? div(n, l) : mk(0.f, 0.f, 0.f);
+    g_sky_faces.edge[f][e] = make_float4(unit.x, unit.y, unit.z, l > 1e-12f ? atan2f(l, dot(u, v)) : 0.0f);
+  }
+}
+
+// Σ coverage x clipped bin weight (sky_face_light, :1489-1498) of sky face f
+// in world axes for horizon n: clipped_bin_weight's values, from the table.
+// Computed bin by bin, the four normalizations and arc tangents of every
+// covered bin took 0.7 of the 6.4 ms of 65,536 receivers' exact sky cones.
+template <class State>
+__device__ __forceinline__ float sky_blocked(State& st, uint32_t f, f3 n) {
+  const float4* corner = g_sky_faces.corner[f];
+  const float4* edge = g_sky_faces.edge[f];
+  auto term = [&](int e) {
+    const float4 t = __ldg(&edge[e]);
+    return t.w * dot(n, xyz(t));
+  };
+  float blocked = 0.0f;
+#pragma unroll 1
+  for (int b = 0; b < kBins; ++b) {
+    const float cv = st.cov_at(b);
+    if (!(cv > 0.0f)) continue;
+    const int col = b % kGrid, row = b / kGrid, p = row * 9 + col;
+    const f3 d0 = xyz(__ldg(&corner[p])), d1 = xyz(__ldg(&corner[p + 1]));
+    const f3 d2 = xyz(__ldg(&corner[p + 10])), d3 = xyz(__ldg(&corner[p + 9]));
+    const int above = (dot(n, d0) > 0.f) + (dot(n, d1) > 0.f) + (dot(n, d2) > 0.f) + (dot(n, d3) > 0.f);
+    float w = 0.0f;
+    // The far edges run against the table's: exact negatives.
+    if (above == 4) w = fabsf(0.5f * (term(b) + term(72 + p + 1) - term(b + 8) - term(72 + p)));
+    else if (above != 0) w = clipped_quad_weight(n, d0, d1, d2, d3);
+    blocked += cv * w;
+  }
+  return blocked;
+}
+
 // The light a light cone's mask lets through (cone_irradiance_rect,
 // :1286-1321: rect lights' Lambert bin weights, one cone at a time across the
 // warp; sphere_open_share, :957-972), times the spot factor, and the lighting
@@ -1442,6 +1504,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, resident_blocks<kWide, kS
     float spot = 1.0f;
     LightConeInfo info{true, false, false};
     bool traced;
+    [[maybe_unused]] bool framed = false;  // a sky face in its object's axes
     if constexpr (kSplit) {
       st.cone = record_cone(rec);
       st.rec = &records[slot_local];
@@ -1465,6 +1528,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, resident_blocks<kWide, kS
           if (x != kNoneU) frame = s.xforms + 4 * (size_t)x;
         }
       }
+      framed = frame != nullptr;
       traced = valid && sky_face(l, point, normal, st.cone, frame);
       st.cap = 0xffffffffu;
       st.independent = (q.sky & kSkyCombineMax) == 0u;
@@ -1517,10 +1581,14 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, resident_blocks<kWide, kS
       if constexpr (!kSplat && !kInst) st.cone = load_cone(ws, table_slot<WS>(lane));
       if (traced) {
         float blocked = 0.0f;
+        if (!framed) {
+          blocked = sky_blocked(st, l, normal);
+        } else {
 #pragma unroll 1
-        for (int b = 0; b < kBins; ++b) {
-          const float cv = st.cov_at(b);
-          if (cv > 0.0f) blocked += cv * clipped_bin_weight(st.cone, normal, b);
+          for (int b = 0; b < kBins; ++b) {
+            const float cv = st.cov_at(b);
+            if (cv > 0.0f) blocked += cv * clipped_bin_weight(st.cone, normal, b);
+          }
         }
         const float open = clipped_window_weight(st.cone, normal);
         value = fmaxf(open - blocked, 0.0f);

@@ -9,6 +9,11 @@ cudaError_t upload_disk_table_splat(const float* table64) {
   return cudaMemcpyToSymbol(c_disk, table64, kBins * sizeof(float));
 }
 
+cudaError_t make_sky_table_splat() {
+  sky_table_kernel<<<6, 160>>>();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_splat_pass(bool wide, bool count, bool inst, bool sky, const DevScene& s, const DevQuery& q,
                               const DevOut& o, const uint32_t* list, const uint32_t* list_count, uint32_t pw,
                               uint32_t blocks, cudaStream_t stream) {
