@@ -36,6 +36,25 @@ constexpr int kBlocksPerSm = 8;
 constexpr int kSoloBlocksPerSm = 8;
 constexpr int kFusedBlocksPerSm = 5;
 constexpr int kFusedSoloBlocksPerSm = 5;
+// Warps per SM the launch rules for small calls aim at: the resident wave of
+// the split packet pass.
+constexpr int kWarpsPerSm = kWarpsPerBlock * kBlocksPerSm;
+// Cones a launch of `cones` walks per packet: at most `most`, halved (down to
+// 2) while the packets would leave resident warps idle: a small call is the
+// time of its heaviest packet. With integrate_slots, host calls of 4,096 cones
+// 468 -> 340 us; 65,536 cones keep packets of 16.
+constexpr uint32_t launch_packet_cones(uint32_t most, uint64_t cones, int sm_count) {
+  while (most > 2 && cones / most < (uint64_t)sm_count * kWarpsPerSm) most = (most + 1) / 2;
+  return most;
+}
+// Slots a warp integrates: 32, halved (down to 4) while the warps would not
+// fill one resident wave (20 per SM; a warp takes its slots' masks one after
+// the other: 4,096 cones took 130 us in 128 warps).
+constexpr uint32_t integrate_slots(uint64_t n, int sm_count) {
+  uint32_t per = 32;
+  while (per > 4 && n / per < (uint64_t)sm_count * 20) per /= 2;
+  return per;
+}
 constexpr int kSkySplatBlocksPerSm = 6;  // prefiltering sky cones' passes (thread-local coverages)
 
 struct DevQuery {
@@ -251,10 +270,10 @@ cudaError_t launch_cone_setup(const DevQuery& q, uint64_t base, uint64_t n, Cone
 constexpr uint32_t kMaxOrderedLights = 1024;
 cudaError_t launch_light_order(const DevQuery& q, uint32_t* out, cudaStream_t stream);
 cudaError_t launch_integrate(const DevQuery& q, const DevOut& o, uint64_t base, uint64_t n, const ConeRecord* records,
-                             cudaStream_t stream);
+                             int sm_count, cudaStream_t stream);
 // Batched: the batch cones of chunk b (b.cone_base .. + b.cone_count).
 cudaError_t launch_batch_setup(const BatchLaunch& b, cudaStream_t stream);
-cudaError_t launch_batch_integrate(const BatchLaunch& b, const DevOut& o, cudaStream_t stream);
+cudaError_t launch_batch_integrate(const BatchLaunch& b, const DevOut& o, int sm_count, cudaStream_t stream);
 
 // The packet pass over every cone, then (with o.redo_list) the solo pass over
 // the cones it listed. o.redo_count and o.error must be zero on entry. Exact

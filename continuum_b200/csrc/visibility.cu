@@ -96,7 +96,7 @@ static cudaError_t split_visibility(const DevScene& s, const DevQuery& q0, const
       e = cudaEventRecord(walked, stream);
       if (e != cudaSuccess) return e;
     }
-    e = launch_integrate(q, o, base, n, q.records, stream);
+    e = launch_integrate(q, o, base, n, q.records, sm_count, stream);
     if (e != cudaSuccess) return e;
   }
   if (marks) cudaEventRecord(marks[2], stream);
@@ -107,8 +107,11 @@ cudaError_t launch_visibility(const DevScene& s, const DevQuery& q, const DevOut
                               uint64_t chunk, int sm_count, cudaStream_t stream, const cudaEvent_t* marks,
                               cudaEvent_t walked) {
   if (pw < 1) pw = 1;
-  pw = packet_cones(pw, q.prefilter > 0.0f || (q.sky & kSkyCones) != 0u);
   const uint64_t ncones = q.npoints * (uint64_t)q.nlights;
+  pw = packet_cones(pw, q.prefilter > 0.0f || (q.sky & kSkyCones) != 0u);
+  // Counting calls keep the packets: their status words say how a cone's
+  // packet walked.
+  if (!count) pw = launch_packet_cones(pw, ncones, sm_count);
   if (ncones == 0) {
     if (marks) {
       cudaEventRecord(marks[0], stream);
@@ -197,7 +200,7 @@ cudaError_t launch_batch(const BatchLaunch& b0, const DevOut& o, const BatchChun
       }
       if (e != cudaSuccess) return e;
     }
-    e = launch_batch_integrate(b, o, stream);
+    e = launch_batch_integrate(b, o, sm_count, stream);
     if (e != cudaSuccess) return e;
   }
   return e;

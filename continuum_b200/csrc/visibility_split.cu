@@ -102,19 +102,19 @@ struct IntegrateShared {
   float scratch[kConeFields * 32];
 };
 
-// One warp per 32 slots (n of them, from slot 0 of the chunk's records and
+// One warp per `per` slots (n of them, from slot 0 of the chunk's records and
 // masks; plain calls with a cone list stop at the list's end): each walked
 // mask integrated as the fused kernels integrate it (light_integral), the
 // results written at each slot's cone, in its job's outputs when batched.
 template <bool kBatch>
 __global__ void __launch_bounds__(64) integrate_kernel(DevQuery q, DevOut o, BatchLaunch b, uint64_t base,
-                                                      uint64_t n, const ConeRecord* __restrict__ records) {
+                                                      uint64_t n, uint32_t per, const ConeRecord* __restrict__ records) {
   __shared__ IntegrateShared sh[2];
   const int lane = threadIdx.x & 31;
   IntegrateShared* ws = sh + (threadIdx.x >> 5);
-  const uint64_t first = ((uint64_t)blockIdx.x * 2 + (threadIdx.x >> 5)) * 32;
+  const uint64_t first = ((uint64_t)blockIdx.x * 2 + (threadIdx.x >> 5)) * per;
   if (first >= n) return;  // the whole warp leaves together
-  uint64_t limit = n;
+  uint64_t limit = first + per < n ? first + per : n;
   if (!kBatch && q.cones) {
     const uint64_t listed = *q.cones_count;
     const uint64_t left = listed > base ? listed - base : 0;
@@ -246,10 +246,11 @@ cudaError_t launch_cone_setup(const DevQuery& q, uint64_t base, uint64_t n, Cone
 }
 
 cudaError_t launch_integrate(const DevQuery& q, const DevOut& o, uint64_t base, uint64_t n,
-                             const ConeRecord* records, cudaStream_t stream) {
+                             const ConeRecord* records, int sm_count, cudaStream_t stream) {
   if (n == 0 || (!o.irradiance && !o.fraction)) return cudaSuccess;
-  const uint64_t warps = (n + 31) / 32;
-  integrate_kernel<false><<<(unsigned)((warps + 1) / 2), 64, 0, stream>>>(q, o, BatchLaunch{}, base, n, records);
+  const uint32_t per = integrate_slots(n, sm_count);
+  const uint64_t warps = (n + per - 1) / per;
+  integrate_kernel<false><<<(unsigned)((warps + 1) / 2), 64, 0, stream>>>(q, o, BatchLaunch{}, base, n, per, records);
   return cudaGetLastError();
 }
 
@@ -260,11 +261,13 @@ cudaError_t launch_batch_setup(const BatchLaunch& b, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_integrate(const BatchLaunch& b, const DevOut& o, cudaStream_t stream) {
+cudaError_t launch_batch_integrate(const BatchLaunch& b, const DevOut& o, int sm_count, cudaStream_t stream) {
   const uint64_t n = b.cone_count;
   if (n == 0) return cudaSuccess;
-  const uint64_t warps = (n + 31) / 32;
-  integrate_kernel<true><<<(unsigned)((warps + 1) / 2), 64, 0, stream>>>(DevQuery{}, o, b, b.cone_base, n, b.records);
+  const uint32_t per = integrate_slots(n, sm_count);
+  const uint64_t warps = (n + per - 1) / per;
+  integrate_kernel<true>
+      <<<(unsigned)((warps + 1) / 2), 64, 0, stream>>>(DevQuery{}, o, b, b.cone_base, n, per, b.records);
   return cudaGetLastError();
 }
 
