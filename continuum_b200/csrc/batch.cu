@@ -72,8 +72,8 @@ int check_options(const cc_batch_options& o) {
 // sizes the device buffers and uploads the job table. The previous
 // submission has finished.
 int prepare(cc_batch* b, uint32_t points_per_warp) {
-  const uint32_t pw = cc::packet_cones(points_per_warp), splat_pw = cc::packet_cones(points_per_warp, true);
-  if (b->prepared && b->prepared_pw == points_per_warp && b->prepared_chunk == b->ctx->split_chunk) return CC_OK;
+  const uint32_t pw = cc::packet_cones(points_per_warp);
+  if (b->prepared && b->prepared_pw == pw && b->prepared_chunk == b->ctx->split_chunk) return CC_OK;
   drop_graph(b);
   uint64_t packet = 0, cone = 0, point = 0;
   std::vector<uint64_t> job_cones;
@@ -125,7 +125,7 @@ int prepare(cc_batch* b, uint32_t points_per_warp) {
       j.packet_start = sp;
       j.cone_start = sc;
       j.point_start = spt;
-      sp += (c + splat_pw - 1) / splat_pw;
+      sp += (c + pw - 1) / pw;
       sc += c;
       spt += j.query.npoints;
     }
@@ -140,7 +140,7 @@ int prepare(cc_batch* b, uint32_t points_per_warp) {
             "batch prefiltering job table upload");
   }
   b->prepared = true;
-  b->prepared_pw = points_per_warp;
+  b->prepared_pw = pw;
   b->prepared_chunk = b->ctx->split_chunk;
   return CC_OK;
 }
@@ -197,7 +197,7 @@ int enqueue(cc_batch* b, const cc_batch_options& opt, cudaStream_t stream) {
     S.njobs = (uint32_t)b->splat_jobs.size();
     S.packets = b->splat_packets;
     S.points = b->splat_points;
-    S.pw = cc::packet_cones(opt.points_per_warp, true);
+    S.pw = cc::packet_cones(opt.points_per_warp);
     S.inst = b->splat_instanced ? 1u : 0u;
     if (!(opt.flags & CC_KEEP_ORDER) && b->splat_points > 0) {
       CC_CUDA(cc::batch_order(S, b->splat_sort_scratch.ptr, b->splat_sort_scratch.size,

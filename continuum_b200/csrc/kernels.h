@@ -14,14 +14,14 @@ constexpr int kWarpsPerBlock = 2;
 // so a packet of 16 keeps the lanes as busy as one of 32, with half the shared
 // memory and half the time of the heaviest packet, which ends the pass: 32, 16
 // and 8 cones took 41.3, 40.2 and 45.3 ms on 3.69 M cones over 3.07 M
-// triangles and 10.7, 7.2 and 5.9 ms on 229 k cones. Sky and prefiltering
-// cones, which integrate their masks in the walk kernel, a lane each, keep 32
-// (exact sky cones: 6.4 ms, 8.3 with 16).
+// triangles and 10.7, 7.2 and 5.9 ms on 229 k cones. Prefiltering cones too
+// (32 and 16 cones: sky 33.6 and 27.0 ms, light 18.6 and 16.3). Exact sky cones
+// keep 32 (4.9 and 5.9 ms): they walk little and integrate a lane each.
 constexpr uint32_t kPacketCones = 16;
-constexpr uint32_t kFusedPacketCones = 32;
-// `fused`: sky or prefiltering cones.
-constexpr uint32_t packet_cones(uint32_t points_per_warp, bool fused = false) {
-  const uint32_t most = fused ? kFusedPacketCones : kPacketCones;
+constexpr uint32_t kSkyPacketCones = 32;
+// `sky`: exact sky cones.
+constexpr uint32_t packet_cones(uint32_t points_per_warp, bool sky = false) {
+  const uint32_t most = sky ? kSkyPacketCones : kPacketCones;
   return points_per_warp < most ? points_per_warp : most;
 }
 // Resident blocks per SM. Passes that keep each cone's coverages in
@@ -34,8 +34,8 @@ constexpr uint32_t packet_cones(uint32_t points_per_warp, bool fused = false) {
 // memory: 5.
 constexpr int kBlocksPerSm = 8;
 constexpr int kSoloBlocksPerSm = 8;
-constexpr int kFusedBlocksPerSm = 5;
-constexpr int kFusedSoloBlocksPerSm = 5;
+constexpr int kFusedBlocksPerSm = 6;
+constexpr int kFusedSoloBlocksPerSm = 6;
 // Warps per SM the launch rules for small calls aim at: the resident wave of
 // the split packet pass.
 constexpr int kWarpsPerSm = kWarpsPerBlock * kBlocksPerSm;

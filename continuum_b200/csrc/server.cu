@@ -328,7 +328,7 @@ struct JobGroup {
 // `status` (kCounterWords). Returns false once it has abandoned the launch.
 bool enqueue_group(cc_server* s, Slot& slot, JobGroup& g, bool splat, cc::JobGpu* staging, uint32_t* status) {
   cudaStream_t st = slot.stream;
-  const uint32_t pw = cc::packet_cones(s->opt.points_per_warp, splat);
+  const uint32_t pw = cc::packet_cones(s->opt.points_per_warp);
   cudaError_t e = cudaSuccess;
   std::memcpy(staging, g.jobs.data(), g.jobs.size() * sizeof(cc::JobGpu));
   const uint64_t sort_bytes = cc::batch_order_scratch_bytes(g.points);
@@ -457,8 +457,7 @@ void launch(cc_server* s, Slot& slot) {
           j.lo[k] = sc->flat.nodes[0].lo[k];
           j.hi[k] = sc->flat.nodes[0].hi[k];
         }
-      const bool prefilter = q.prefilter > 0.0f;
-      (prefilter ? splat : exact).add(j, P, cc::packet_cones(s->opt.points_per_warp, prefilter));
+      (q.prefilter > 0.0f ? splat : exact).add(j, P, cc::packet_cones(s->opt.points_per_warp));
       ++t;
     }
   }

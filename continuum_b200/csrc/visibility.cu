@@ -108,7 +108,7 @@ cudaError_t launch_visibility(const DevScene& s, const DevQuery& q, const DevOut
                               cudaEvent_t walked) {
   if (pw < 1) pw = 1;
   const uint64_t ncones = q.npoints * (uint64_t)q.nlights;
-  pw = packet_cones(pw, q.prefilter > 0.0f || (q.sky & kSkyCones) != 0u);
+  pw = packet_cones(pw, (q.sky & kSkyCones) != 0u && !(q.prefilter > 0.0f));
   // Counting calls keep the packets: their status words say how a cone's
   // packet walked.
   if (!count) pw = launch_packet_cones(pw, ncones, sm_count);

@@ -100,7 +100,7 @@ template <bool kWide, bool kSky, bool kSplat, bool kBack = false, bool kInst = f
 using KernelShared = typename std::conditional<
     kWide, WarpShared<unsigned long long, kSky, smem_cov<kSky, kSplat>(), kBack, kInst, 1, kSplat>,
     WarpShared<unsigned int, kSky, smem_cov<kSky, kSplat>(), kBack, kInst,
-               (int)(kSky || kSplat ? kFusedPacketCones : kPacketCones), kSplat>>::type;
+               (int)(kSky && !kSplat ? kSkyPacketCones : kPacketCones), kSplat>>::type;
 constexpr int resident_blocks_for(bool wide, bool sky, bool splat) {
   return (splat && !sky) ? (wide ? kFusedSoloBlocksPerSm : kFusedBlocksPerSm)
                          : (splat ? kSkySplatBlocksPerSm : (wide ? kSoloBlocksPerSm : kBlocksPerSm));
