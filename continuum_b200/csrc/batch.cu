@@ -396,10 +396,7 @@ int add_job(cc_batch* b, const cc_scene* scene, const float* receivers, uint64_t
   j.fraction = out->fraction;
   j.work = reinterpret_cast<uint4*>(out->work);
   if (!scene->flat.nodes.empty()) {
-    for (int k = 0; k < 3; ++k) {
-      j.lo[k] = scene->flat.nodes[0].lo[k];
-      j.hi[k] = scene->flat.nodes[0].hi[k];
-    }
+    j.grid = cc::grid_over(scene->flat.nodes[0].lo, scene->flat.nodes[0].hi);
   }
   if (job) *job = (uint32_t)(b->jobs.size() + b->splat_jobs.size());
   b->count_work = b->count_work || out->work != nullptr;

@@ -24,14 +24,12 @@ constexpr uint32_t packet_cones(uint32_t points_per_warp, bool sky = false) {
   const uint32_t most = sky ? kSkyPacketCones : kPacketCones;
   return points_per_warp < most ? points_per_warp : most;
 }
-// Resident blocks per SM. Passes that keep each cone's coverages in
-// thread-local memory (the split path's, exact sky cones') take 8: 128
-// registers a thread, and 16 KB of shared memory per block in the packet pass
-// (27 KB for sky cones; the solo pass holds one cone's cells, 6 KB). 10 and 12
-// blocks (96 and 80 registers, with spills) ran the same: instruction fetch,
-// not the warps in flight, is the bound. Prefiltering sky cones, whose walk needs more
-// registers, take 6. Prefiltering light cones keep their coverages in shared
-// memory: 5.
+// Resident blocks per SM. Exact cones' passes take 8: 128 registers a thread,
+// and 16 KB of shared memory per block in the packet pass (32-bit accumulator
+// cells of 16 cones; 27 KB for sky cones; the solo pass holds one cone's
+// cells, 6 KB). 10 and 12 blocks (96 and 80 registers, with spills) ran the
+// same: instruction fetch, not the warps in flight, is the bound.
+// Prefiltering cones, whose walk needs 168 registers, take 6.
 constexpr int kBlocksPerSm = 8;
 constexpr int kSoloBlocksPerSm = 8;
 constexpr int kFusedBlocksPerSm = 6;
@@ -162,6 +160,19 @@ struct DevOut {
 // Scratch words per call: redo count, error word, packet and solo counters.
 constexpr int kCounterWords = 4;
 
+// A point's code: its cell on a grid of cubes over the scene's bounds, the
+// cells' bits interleaved from the longest axis's highest down, kCodeBits in
+// all. Cubes, because a packet's cones should start close together: with ten
+// bits to each axis whatever its length, a field 2 km wide and 6 m high had
+// cells of 2 m x 6 mm x 2 m, and a packet on a sphere was a contour line.
+constexpr int kCodeBits = 32;
+struct OrderGrid {
+  float lo[3] = {0.f, 0.f, 0.f};
+  float inv = 0.f;  // 1 / the cell's side
+  int bits[3] = {0, 0, 0};
+};
+OrderGrid grid_over(const float* lo, const float* hi);
+
 // One job of a batch: its scene, query and outputs, and where its packets,
 // cones and points start in the batch's numbering. A batch's packets never
 // straddle two jobs.
@@ -177,7 +188,7 @@ struct JobGpu {
   uint64_t packet_start;
   uint64_t cone_start;
   uint64_t point_start;
-  float lo[3], hi[3];  // the scene's bounds (Morton quantization)
+  OrderGrid grid;  // over the scene's bounds
 };
 
 // A batch launch: the job table and the batch's sizes. The redo list and
@@ -214,7 +225,7 @@ struct BatchChunk {
 std::vector<BatchChunk> batch_chunks(const std::vector<uint64_t>& cones, uint32_t pw, uint64_t max_slots);
 
 // Morton walk order of every job's points in one sort: keys are the job index
-// above each point's 30-bit code, values the job-local point index; job j's
+// above each point's code, values the job-local point index; job j's
 // order lands at order + jobs[j].point_start.
 size_t batch_order_scratch_bytes(uint64_t points);
 cudaError_t batch_order(const BatchLaunch& b, void* scratch, size_t scratch_bytes, uint32_t* order,

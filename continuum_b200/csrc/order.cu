@@ -3,8 +3,8 @@
 // A warp walks up to 32 cones together and visits the union of the nodes
 // its cones need, so cones in a warp should see the same geometry. Callers
 // list receivers in their own order (image rows, texels of many pages); here
-// each receiver gets a 30-bit Morton code of its position quantized in the
-// scene's bounds, and a device radix sort yields the walk order. Results do
+// each receiver gets a Morton code of its position quantized in the scene's
+// bounds, and a device radix sort yields the walk order. Results do
 // not depend on the order — only which cones share a warp.
 #include <cub/device/device_radix_sort.cuh>
 
@@ -16,32 +16,35 @@ namespace cc {
 
 namespace {
 
-__device__ __forceinline__ uint32_t spread10(uint32_t v) {
-  v &= 0x3ffu;
-  v = (v | (v << 16)) & 0x030000ffu;
-  v = (v | (v << 8)) & 0x0300f00fu;
-  v = (v | (v << 4)) & 0x030c30c3u;
-  v = (v | (v << 2)) & 0x09249249u;
-  return v;
+__device__ __forceinline__ uint32_t grid_code(const OrderGrid& g, float4 p) {
+  const float x[3] = {p.x, p.y, p.z};
+  uint32_t c[3];
+  int top = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float most = (float)((1u << g.bits[k]) - 1u);
+    c[k] = (uint32_t)fminf(fmaxf((x[k] - g.lo[k]) * g.inv, 0.0f), most);  // NaN clamps to 0
+    top = max(top, g.bits[k]);
+  }
+  uint32_t code = 0;
+  for (int b = top - 1; b >= 0; --b) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (b < g.bits[k]) code = (code << 1) | ((c[k] >> b) & 1u);
+  }
+  return code;
 }
 
-__global__ void morton_keys(const float4* __restrict__ receivers, uint64_t n, float3 lo, float3 scale,
-                            uint32_t* __restrict__ keys, uint32_t* __restrict__ index) {
+__global__ void morton_keys(const float4* __restrict__ receivers, uint64_t n, OrderGrid grid, uint32_t* __restrict__ keys,
+                            uint32_t* __restrict__ index) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float4 p = __ldg(&receivers[2 * i]);
-  auto q = [](float x, float l, float s) {
-    float t = (x - l) * s;
-    t = fminf(fmaxf(t, 0.0f), 1023.0f);  // NaN clamps to 0
-    return (uint32_t)t;
-  };
-  keys[i] = (spread10(q(p.x, lo.x, scale.x)) << 2) | (spread10(q(p.y, lo.y, scale.y)) << 1) |
-            spread10(q(p.z, lo.z, scale.z));
+  keys[i] = grid_code(grid, __ldg(&receivers[2 * i]));
   index[i] = (uint32_t)i;
 }
 
-// Batch keys: the job's index above the point's 30-bit code; values: the
-// point's index within its job.
+// Batch keys: the job's index above the point's code; values: the point's
+// index within its job.
 __global__ void batch_morton_keys(BatchLaunch b, unsigned long long* __restrict__ keys,
                                   uint32_t* __restrict__ index) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -53,16 +56,7 @@ __global__ void batch_morton_keys(BatchLaunch b, unsigned long long* __restrict_
   }
   const JobGpu& J = b.jobs[lo];
   const uint64_t local = i - J.point_start;
-  const float4 p = __ldg(&J.query.receivers[2 * local]);
-  auto q = [](float x, float l, float h) {
-    const float s = (h - l) > 0.0f ? 1023.0f / (h - l) : 0.0f;
-    float t = (x - l) * s;
-    t = fminf(fmaxf(t, 0.0f), 1023.0f);  // NaN clamps to 0
-    return (uint32_t)t;
-  };
-  const uint32_t code = (spread10(q(p.x, J.lo[0], J.hi[0])) << 2) | (spread10(q(p.y, J.lo[1], J.hi[1])) << 1) |
-                        spread10(q(p.z, J.lo[2], J.hi[2]));
-  keys[i] = ((unsigned long long)lo << 30) | code;
+  keys[i] = ((unsigned long long)lo << kCodeBits) | grid_code(J.grid, __ldg(&J.query.receivers[2 * local]));
   index[i] = (uint32_t)local;
 }
 
@@ -73,6 +67,35 @@ int job_bits(uint32_t njobs) {
 }
 
 }  // namespace
+
+OrderGrid grid_over(const float* lo, const float* hi) {
+  OrderGrid g;
+  float e[3], longest = 0.0f;
+  for (int k = 0; k < 3; ++k) {
+    g.lo[k] = lo[k];
+    e[k] = hi[k] - lo[k];
+    if (!(e[k] > 0.0f)) e[k] = 0.0f;
+    longest = e[k] > longest ? e[k] : longest;
+    g.bits[k] = 0;
+  }
+  g.inv = 0.0f;
+  if (!(longest > 0.0f) || !(longest < 1e30f)) return g;
+  // Halve the cell from the longest axis's length while the codes fit.
+  float side = longest;
+  for (;;) {
+    int bits[3], sum = 0;
+    for (int k = 0; k < 3; ++k) {
+      bits[k] = 0;
+      while (bits[k] < kCodeBits && side * 0.5f * (float)(1u << bits[k]) < e[k] && bits[k] < 31) ++bits[k];
+      sum += bits[k];
+    }
+    if (sum > kCodeBits || bits[0] > 20 || bits[1] > 20 || bits[2] > 20) break;
+    for (int k = 0; k < 3; ++k) g.bits[k] = bits[k];
+    side *= 0.5f;
+  }
+  g.inv = 1.0f / side;
+  return g;
+}
 
 size_t batch_order_scratch_bytes(uint64_t points) {
   size_t temp = 0;
@@ -102,13 +125,13 @@ cudaError_t batch_order(const BatchLaunch& b, void* scratch, size_t scratch_byte
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_in, keys_out, idx_in, order, (int)n, 0,
-                                         30 + job_bits(b.njobs), stream);
+                                         kCodeBits + job_bits(b.njobs), stream);
 }
 
 size_t walk_order_scratch_bytes(uint64_t npoints) {
   size_t temp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, temp, (const uint32_t*)nullptr, (uint32_t*)nullptr,
-                                  (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)npoints, 0, 30);
+                                  (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)npoints, 0, kCodeBits);
   return 4 * npoints * sizeof(uint32_t) + temp + 256;
 }
 
@@ -124,16 +147,14 @@ cudaError_t walk_order(const float4* receivers, uint64_t npoints, const float* s
   const size_t used = static_cast<size_t>(temp - static_cast<uint8_t*>(scratch));
   if (used > scratch_bytes) return cudaErrorInvalidValue;
   size_t temp_bytes = scratch_bytes - used;
-  float3 lo = make_float3(scene_lo[0], scene_lo[1], scene_lo[2]);
-  auto inv = [](float a, float b) { return (b - a) > 0.0f ? 1023.0f / (b - a) : 0.0f; };
-  float3 scale = make_float3(inv(scene_lo[0], scene_hi[0]), inv(scene_lo[1], scene_hi[1]), inv(scene_lo[2], scene_hi[2]));
+  const OrderGrid grid = grid_over(scene_lo, scene_hi);
   const unsigned threads = 256;
   const unsigned blocks = (unsigned)((npoints + threads - 1) / threads);
-  morton_keys<<<blocks, threads, 0, stream>>>(receivers, npoints, lo, scale, keys_in, idx_in);
+  morton_keys<<<blocks, threads, 0, stream>>>(receivers, npoints, grid, keys_in, idx_in);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  return cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_in, keys_out, idx_in, order, (int)npoints, 0, 30,
-                                         stream);
+  return cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_in, keys_out, idx_in, order, (int)npoints, 0,
+                                         max(grid.bits[0] + grid.bits[1] + grid.bits[2], 1), stream);
 }
 
 }  // namespace cc

@@ -453,10 +453,7 @@ void launch(cc_server* s, Slot& slot) {
       j.irradiance = reinterpret_cast<float*>(block + 16 * P);
       j.fraction = reinterpret_cast<float*>(block + 20 * P);
       if (!sc->flat.nodes.empty())
-        for (int k = 0; k < 3; ++k) {
-          j.lo[k] = sc->flat.nodes[0].lo[k];
-          j.hi[k] = sc->flat.nodes[0].hi[k];
-        }
+        j.grid = cc::grid_over(sc->flat.nodes[0].lo, sc->flat.nodes[0].hi);
       (q.prefilter > 0.0f ? splat : exact).add(j, P, cc::packet_cones(s->opt.points_per_warp));
       ++t;
     }

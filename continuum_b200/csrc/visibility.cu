@@ -41,7 +41,7 @@ cudaError_t upload_disk_table(const float* table64) {
   sky_table_kernel<<<6, 160>>>();
   e = cudaGetLastError();
   if (e == cudaSuccess) e = make_sky_table_splat();
-  return e == cudaSuccess ? cudaDeviceSynchronize() : e;
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
 }
 
 // The exact cones' plain pass (packet or solo) of the variant the flags pick;
