@@ -83,15 +83,11 @@ int upload(const std::vector<T>& host, T** dev, uint64_t& bytes, const char* wha
 }
 
 void free_scene_device(cc_scene* s) {
-  cudaFree(s->tris);
-  cudaFree(s->meshes);
-  cudaFree(s->nodes);
-  cudaFree(s->items);
-  cudaFree(s->blas);
-  cudaFree(s->xforms);
+  cudaFree(s->block);  // the arrays of upload_scene
   cudaFree(s->blas_cov);
   cudaFree(s->obj_cov);
   cudaFree(s->tri_slot);
+  s->block = nullptr;
   s->tri_slot = nullptr;
   s->blas_cov = nullptr;
   s->obj_cov = nullptr;
@@ -124,18 +120,43 @@ int upload_scene(cc_scene* s) {
   // Without meshes the object hierarchy is one leaf holding mesh 0, which
   // must then be an empty range (as flatten pads it, hierarchy.rs:57-59).
   if (meshes.empty()) meshes.push_back(make_uint4(0u, 0u, CC_NONE, CC_NONE));
-  int rc;
-  if ((rc = upload(tris, &s->tris, s->bytes, "scene triangles"))) return rc;
-  if ((rc = upload(meshes, &s->meshes, s->bytes, "scene meshes"))) return rc;
-  if ((rc = upload(repack(f.nodes), &s->nodes, s->bytes, "scene nodes"))) return rc;
-  if ((rc = upload(f.items, &s->items, s->bytes, "scene items"))) return rc;
-  if ((rc = upload(repack(f.blas), &s->blas, s->bytes, "scene triangle nodes"))) return rc;
-  if (!f.xforms.empty()) {
-    std::vector<float4> x(f.xforms.size() / 4);
-    for (size_t i = 0; i < x.size(); ++i)
-      x[i] = make_float4(f.xforms[4 * i], f.xforms[4 * i + 1], f.xforms[4 * i + 2], f.xforms[4 * i + 3]);
-    if ((rc = upload(x, &s->xforms, s->bytes, "scene transforms"))) return rc;
+  const std::vector<float4> nodes = repack(f.nodes), blas = repack(f.blas);
+  std::vector<float4> xforms(f.xforms.size() / 4);
+  for (size_t i = 0; i < xforms.size(); ++i)
+    xforms[i] = make_float4(f.xforms[4 * i], f.xforms[4 * i + 1], f.xforms[4 * i + 2], f.xforms[4 * i + 3]);
+  // One allocation for the scene, and for a small one a single copy: six of
+  // each (and of the frees) made most of a call that brings its meshes along.
+  struct Part {
+    const void* host;
+    size_t bytes, at;
+    void** dev;
+  };
+  Part parts[] = {{tris.data(), tris.size() * sizeof(float4), 0, reinterpret_cast<void**>(&s->tris)},
+                  {meshes.data(), meshes.size() * sizeof(uint4), 0, reinterpret_cast<void**>(&s->meshes)},
+                  {nodes.data(), nodes.size() * sizeof(float4), 0, reinterpret_cast<void**>(&s->nodes)},
+                  {f.items.data(), f.items.size() * sizeof(uint32_t), 0, reinterpret_cast<void**>(&s->items)},
+                  {blas.data(), blas.size() * sizeof(float4), 0, reinterpret_cast<void**>(&s->blas)},
+                  {xforms.data(), xforms.size() * sizeof(float4), 0, reinterpret_cast<void**>(&s->xforms)}};
+  size_t total = 0;
+  for (Part& p : parts) {
+    p.at = total;
+    total += (std::max<size_t>(p.bytes, 16) + 255) & ~size_t(255);
   }
+  CC_CUDA(cudaMalloc(&s->block, total), "scene arrays");
+  uint8_t* base = static_cast<uint8_t*>(s->block);
+  for (const Part& p : parts)
+    if (p.bytes || p.dev != reinterpret_cast<void**>(&s->xforms)) *p.dev = base + p.at;  // no transforms: null
+  constexpr size_t kStaged = size_t(1) << 20;
+  if (total <= kStaged) {
+    std::vector<uint8_t> staged(total, 0);
+    for (const Part& p : parts)
+      if (p.bytes) std::memcpy(&staged[p.at], p.host, p.bytes);
+    CC_CUDA(cudaMemcpy(base, staged.data(), total, cudaMemcpyHostToDevice), "scene arrays");
+  } else {
+    for (const Part& p : parts)
+      if (p.bytes) CC_CUDA(cudaMemcpy(base + p.at, p.host, p.bytes, cudaMemcpyHostToDevice), "scene arrays");
+  }
+  s->bytes += total;
   return CC_OK;
 }
 
@@ -969,18 +990,15 @@ int cc_irradiance(cc_context* ctx, const float* receivers6, uint64_t npoints, co
   opt.hierarchy = hierarchy;
   opt.flags = CC_DEVICE_POINTERS;
   // Inputs and the output on the device, then `runs` timed executions.
-  float4* d_rec = nullptr;
-  float4* d_light = nullptr;
-  float* d_out = nullptr;
-  auto cleanup = [&] {
-    cudaFree(d_rec);
-    cudaFree(d_light);
-    cudaFree(d_out);
-    cc_scene_destroy(scene);
-  };
-  cudaError_t e = cudaMalloc(&d_rec, std::max<uint64_t>(npoints, 1) * 32);
-  if (e == cudaSuccess) e = cudaMalloc(&d_light, 64);
-  if (e == cudaSuccess) e = cudaMalloc(&d_out, std::max<uint64_t>(npoints, 1) * 4);
+  // (in the context's buffers: its calls with device pointers use none of
+  // the three).
+  auto cleanup = [&] { cc_scene_destroy(scene); };
+  cudaError_t e = ctx->receivers.reserve(std::max<uint64_t>(npoints, 1) * 32);
+  if (e == cudaSuccess) e = ctx->lights.reserve(64);
+  if (e == cudaSuccess) e = ctx->irradiance.reserve(std::max<uint64_t>(npoints, 1) * 4);
+  float4* d_rec = static_cast<float4*>(ctx->receivers.ptr);
+  float4* d_light = static_cast<float4*>(ctx->lights.ptr);
+  float* d_out = static_cast<float*>(ctx->irradiance.ptr);
   if (e == cudaSuccess && npoints) e = cudaMemcpy(d_rec, rec.data(), npoints * 32, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d_light, light, 64, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {

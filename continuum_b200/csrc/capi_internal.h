@@ -93,6 +93,7 @@ struct cc_context {
 struct cc_scene {
   cc_context* ctx = nullptr;
   cc::FlatScene flat;  // host copy of the reference layouts
+  void* block = nullptr;  // one allocation: tris, meshes, nodes, items, blas, xforms
   float4* tris = nullptr;
   uint4* meshes = nullptr;
   float4* nodes = nullptr;
