@@ -80,3 +80,35 @@ def test_few_cones(kernel):
     meshes, lights, rec = sliced_scene([1280])
     same(kernel, meshes, lights[:1], rec[:1])
     same(kernel, meshes, lights, rec[:33])
+
+
+@pytest.mark.parametrize("n", [1, 65, 4735, 4737, 37889])
+def test_small_calls_packets_change_no_result(kernel, n):
+    """Small calls walk and integrate in smaller pieces; calls that count work
+    keep the packets, so they give the other side."""
+    meshes, lights, rec = sliced_scene([300, 40])
+    rec = np.ascontiguousarray(np.tile(rec, (n // len(rec) + 1, 1))[:n])
+    scene = kernel.scene(meshes)
+    a = kernel.visibility(scene, rec, lights)
+    b = kernel.visibility(scene, rec, lights, outputs=ALL)
+    scene.close()
+    for k in ("full", "any", "irradiance", "fraction"):
+        assert np.array_equal(getattr(a, k), getattr(b, k)), k
+
+
+@pytest.mark.parametrize("squeeze", [(1, 1, 1), (1, 0, 1), (0, 1, 0), (1e-3, 1, 40)])
+def test_walk_order_over_any_bounds(kernel, squeeze):
+    """The walk order's grid over flat and long scenes, receivers outside their
+    bounds and receivers that are no numbers: the order changes no result."""
+    from continuum_b200 import _lib
+
+    meshes, lights, rec = sliced_scene([200, 64])
+    meshes = [np.ascontiguousarray(m * np.asarray(squeeze, np.float32)) for m in meshes]
+    rec[::50, 0:3] *= 1e3
+    rec[7::100, 1] = np.nan
+    scene = kernel.scene(meshes)
+    a = kernel.visibility(scene, rec, lights)
+    b = kernel.visibility(scene, rec, lights, flags=_lib.CC_KEEP_ORDER)
+    scene.close()
+    for k in ("full", "any", "irradiance", "fraction"):
+        assert np.array_equal(getattr(a, k), getattr(b, k), equal_nan=k in ("irradiance", "fraction")), k
