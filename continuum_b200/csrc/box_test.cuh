@@ -18,13 +18,12 @@ __device__ __forceinline__ bool in_bound(const Cone& c, f3 p, float r) {  // :15
 // kHorizon: sky cones, whose horizon `horizon` (the receiver's normal, in the
 // cone's space) also culls a box wholly below it (:245); a light cone's
 // horizon is zero (:146-147), which culls nothing, so light cones skip it.
-// kUnrolled: the eight corners side by side (the walk's hot test of a node's
-// children); else one at a time, in a fifth of the code (the tests of a
-// walk's root and of meshes' roots, which run far less often).
-template <bool kHorizon = false, bool kUnrolled = true>
+// One corner at a time, in a fifth of the unrolled code: it runs where
+// box_verdict leaves a box open.
+template <bool kHorizon = false>
 __device__ __forceinline__ bool may_touch_box(const Cone& c, f3 lo, f3 hi, f3 horizon = f3{0.f, 0.f, 0.f}) {
   bool far_out = true, near_out = true, out_u0 = true, out_u1 = true, out_v0 = true, out_v1 = true, below = kHorizon;
-#pragma unroll (kUnrolled ? 8 : 1)
+#pragma unroll 1
   for (int k = 0; k < 8; ++k) {
     f3 corner = mk((k & 1) ? hi.x : lo.x, (k & 2) ? hi.y : lo.y, (k & 4) ? hi.z : lo.z);
     if (c.far_offset - dot(c.fwd, corner) >= 0.0f) far_out = false;
@@ -45,7 +44,7 @@ __device__ __forceinline__ bool may_touch_box(const Cone& c, f3 lo, f3 hi, f3 ho
 // may_touch_box decided from a box's centre and half extents. Its exact form
 // asks, plane by plane, whether some corner of eight passes; the plane's
 // largest value over the box is its value at the centre plus |normal| x half
-// extents, a fourteenth of the work. Both are f32 evaluations of one real
+// extents, a quarter of the work. Both are f32 evaluations of one real
 // number with errors below 16 units in the last place of the terms they sum
 // (coordinates from the apex, of size `reach`, times 1 + the window's largest
 // side; for the far plane and the bounding cone, world coordinates), so a
@@ -113,6 +112,6 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
 template <bool kHorizon>
 __device__ __forceinline__ bool touches_box(const Cone& c, const BoxTest& t, f3 lo, f3 hi, f3 horizon) {
   int v = box_verdict<kHorizon>(c, t, lo, hi, horizon);
-  if (v == 2) v = may_touch_box<kHorizon, false>(c, lo, hi, horizon) ? 1 : 0;
+  if (v == 2) v = may_touch_box<kHorizon>(c, lo, hi, horizon) ? 1 : 0;
   return v == 1;
 }

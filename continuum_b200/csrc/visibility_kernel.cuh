@@ -120,22 +120,17 @@ static_assert(shared_fits<false, false, true>() && shared_fits<true, false, true
 static_assert(shared_fits<false, true, true>() && shared_fits<true, true, true>(), "prefiltering sky passes");
 constexpr uint32_t kStatusAccOverflow = 32u;
 
-// A stack entry packed in one word: its kind in the top 2 bits (an
-// object-hierarchy node, a triangle-hierarchy node, or a mesh's resolve
-// marker), then a node's item count in 4 bits (0: interior), then its first
-// item (leaf) or left child (interior) in 26 bits. Each lane keeps two bits
-// per entry: whether its own walk needs the entry, and whether its cone
-// passed the entry's box test, which is done when the parent is visited (the
-// two children of a node are adjacent, so one 64-byte load serves both
-// tests and the nearest-first choice).
+// An exact walk's stack entry packed in one word: a node's item count in 4 bits
+// (0: interior), then its first item (leaf) or left child (interior) in 26
+// bits. Each lane keeps two bits per entry: whether its own walk needs the
+// entry, and whether its cone passed the entry's box test, which is done when
+// the parent is visited (the two children of a node are adjacent, so one
+// 64-byte load serves both tests and the nearest-first choice).
 constexpr uint32_t kRefIndexBits = 26;
 constexpr uint32_t kRefIndexMask = (1u << kRefIndexBits) - 1u;
-constexpr uint32_t kRefKindShift = 30;
-__device__ __forceinline__ uint32_t node_ref(float4 a, float4 b, uint32_t kind) {
-  return (kind << kRefKindShift) | ((__float_as_uint(b.w) & 15u) << kRefIndexBits) |
-         (__float_as_uint(a.w) & kRefIndexMask);
+__device__ __forceinline__ uint32_t node_ref(float4 a, float4 b) {
+  return ((__float_as_uint(b.w) & 15u) << kRefIndexBits) | (__float_as_uint(a.w) & kRefIndexMask);
 }
-__device__ __forceinline__ uint32_t ref_kind(uint32_t r) { return r >> kRefKindShift; }
 __device__ __forceinline__ uint32_t ref_count(uint32_t r) { return (r >> kRefIndexBits) & 15u; }
 __device__ __forceinline__ uint32_t ref_index(uint32_t r) { return r & kRefIndexMask; }
 
@@ -518,9 +513,6 @@ __device__ __forceinline__ void resolve_mesh(const DevScene& s, LaneState<WS>& s
   }
   __syncwarp();
 }
-
-// Stack entry kinds for the walk of both hierarchy levels in one loop.
-constexpr uint32_t kObjNode = 0;   // an object-hierarchy node
 
 // add_mesh_coverage_if (:713-829) for hierarchy levels 0 and 1: every
 // triangle of mesh m for the lanes with `on`, in leaf-sized groups, then the
@@ -967,7 +959,7 @@ __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy
   const float4 ra = __ldg(&s.nodes[0]);
   const float4 rb = __ldg(&s.nodes[1]);
   const bool root_pass = traced && box_in_table(st.ws, own, node_lo(ra), node_lo(rb));
-  stk.push(0, node_ref(ra, rb, kObjNode), traced, root_pass, lane);
+  stk.push(0, node_ref(ra, rb), traced, root_pass, lane);
   int sp = 1;
   while (sp > 0) {
     --sp;
@@ -1038,7 +1030,7 @@ __device__ __forceinline__ void scene_walk(const DevScene& s, uint32_t hierarchy
         if (descend) st.status |= 2u;
         continue;
       }
-      const uint32_t rl = node_ref(la, lb, kObjNode), rr = node_ref(xa, xb, kObjNode);
+      const uint32_t rl = node_ref(la, lb), rr = node_ref(xa, xb);
       // The child popped second below the one popped first.
       stk.push(sp, swap ? rl : rr, descend, swap ? pl : pr, lane);
       stk.push(sp + 1, swap ? rr : rl, descend, swap ? pr : pl, lane);
