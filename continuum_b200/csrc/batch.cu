@@ -116,8 +116,7 @@ int prepare(cc_batch* b, uint32_t points_per_warp) {
   CC_CUDA(b->sort_scratch.reserve(cc::batch_order_scratch_bytes(std::max<uint64_t>(point, 1))), "batch sort scratch");
   CC_CUDA(b->counters.reserve(2 * cc::kCounterWords * sizeof(uint32_t)), "batch counters");
   if (!b->jobs.empty())
-    CC_CUDA(cudaMemcpy(b->job_table.ptr, b->jobs.data(), b->jobs.size() * sizeof(cc::JobGpu), cudaMemcpyHostToDevice),
-            "batch job table upload");
+    CC_CUDA(copy_in(b->job_table.ptr, b->jobs.data(), b->jobs.size() * sizeof(cc::JobGpu)), "batch job table upload");
   if (!b->splat_jobs.empty()) {
     uint64_t sp = 0, sc = 0, spt = 0;
     for (cc::JobGpu& j : b->splat_jobs) {
@@ -135,8 +134,7 @@ int prepare(cc_batch* b, uint32_t points_per_warp) {
     CC_CUDA(b->splat_order.reserve(std::max<uint64_t>(spt, 1) * 4), "batch prefiltering walk order");
     CC_CUDA(b->splat_sort_scratch.reserve(cc::batch_order_scratch_bytes(std::max<uint64_t>(spt, 1))),
             "batch prefiltering sort scratch");
-    CC_CUDA(cudaMemcpy(b->splat_table.ptr, b->splat_jobs.data(), b->splat_jobs.size() * sizeof(cc::JobGpu),
-                       cudaMemcpyHostToDevice),
+    CC_CUDA(copy_in(b->splat_table.ptr, b->splat_jobs.data(), b->splat_jobs.size() * sizeof(cc::JobGpu)),
             "batch prefiltering job table upload");
   }
   b->prepared = true;

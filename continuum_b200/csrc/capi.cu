@@ -77,7 +77,7 @@ template <class T>
 int upload(const std::vector<T>& host, T** dev, uint64_t& bytes, const char* what) {
   size_t n = std::max<size_t>(host.size(), 1) * sizeof(T);
   CC_CUDA(cudaMalloc(dev, n), what);
-  if (!host.empty()) CC_CUDA(cudaMemcpy(*dev, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice), what);
+  if (!host.empty()) CC_CUDA(copy_in(*dev, host.data(), host.size() * sizeof(T)), what);
   bytes += n;
   return CC_OK;
 }
@@ -156,6 +156,7 @@ int upload_scene(cc_scene* s) {
     for (const Part& p : parts)
       if (p.bytes) CC_CUDA(cudaMemcpy(base + p.at, p.host, p.bytes, cudaMemcpyHostToDevice), "scene arrays");
   }
+  CC_CUDA(copies_landed(), "scene arrays");
   s->bytes += total;
   return CC_OK;
 }
@@ -770,19 +771,16 @@ int cc_scene_set_clear(cc_scene* s, const float* clear, uint32_t nobjects) {
   if (!s->ctx) return CC_OK;
   int rc = set_device(s->ctx);
   if (rc) return rc;
-  CC_CUDA(cudaMemcpy(s->xforms, f.xforms.data(), f.xforms.size() * sizeof(float), cudaMemcpyHostToDevice),
-          "object transforms");
+  CC_CUDA(copy_in(s->xforms, f.xforms.data(), f.xforms.size() * sizeof(float)), "object transforms");
   if (s->coverage_ready) {
     // The prefiltered cones' samples scale with the objects' opacity: the
     // same buffers, refilled.
     const std::vector<float> blas = cc::blas_coverage(f);
     if (!blas.empty())
-      CC_CUDA(cudaMemcpy(s->blas_cov, blas.data(), blas.size() * sizeof(float), cudaMemcpyHostToDevice),
-              "triangle-node coverage");
+      CC_CUDA(copy_in(s->blas_cov, blas.data(), blas.size() * sizeof(float)), "triangle-node coverage");
     const std::vector<float> obj = cc::object_coverage(f, blas);
     if (!obj.empty() && s->obj_cov)
-      CC_CUDA(cudaMemcpy(s->obj_cov, obj.data(), obj.size() * sizeof(float), cudaMemcpyHostToDevice),
-              "object-node coverage");
+      CC_CUDA(copy_in(s->obj_cov, obj.data(), obj.size() * sizeof(float)), "object-node coverage");
   }
   return CC_OK;
 }
@@ -989,9 +987,9 @@ int cc_irradiance(cc_context* ctx, const float* receivers6, uint64_t npoints, co
   cc_options_default(&opt);
   opt.hierarchy = hierarchy;
   opt.flags = CC_DEVICE_POINTERS;
-  // Inputs and the output on the device, then `runs` timed executions.
-  // (in the context's buffers: its calls with device pointers use none of
-  // the three).
+  // Inputs and the output on the device, then `runs` timed executions; in the
+  // context's buffers, as one call at a time runs on a context, and copied in
+  // its stream, ahead of the kernels that read them.
   auto cleanup = [&] { cc_scene_destroy(scene); };
   cudaError_t e = ctx->receivers.reserve(std::max<uint64_t>(npoints, 1) * 32);
   if (e == cudaSuccess) e = ctx->lights.reserve(64);
@@ -999,8 +997,9 @@ int cc_irradiance(cc_context* ctx, const float* receivers6, uint64_t npoints, co
   float4* d_rec = static_cast<float4*>(ctx->receivers.ptr);
   float4* d_light = static_cast<float4*>(ctx->lights.ptr);
   float* d_out = static_cast<float*>(ctx->irradiance.ptr);
-  if (e == cudaSuccess && npoints) e = cudaMemcpy(d_rec, rec.data(), npoints * 32, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(d_light, light, 64, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && npoints)
+    e = cudaMemcpyAsync(d_rec, rec.data(), npoints * 32, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_light, light, 64, cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) {
     cleanup();
     return cuda_fail(e, "irradiance inputs");

@@ -47,6 +47,16 @@ struct DevBuf {
 
 int set_device(cc_context* ctx);
 
+// Waits until the copies put in the legacy stream are on the device. A
+// cudaMemcpy from pageable memory may return before that, and the contexts',
+// batches' and servers' streams (non-blocking) do not wait for the legacy
+// stream: every such copy ends with this before its bytes are handed out.
+inline cudaError_t copies_landed() { return cudaStreamSynchronize(nullptr); }
+inline cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? copies_landed() : e;
+}
+
 // cc_visibility's body (capi.cu): `sky` makes the cones sky faces (0: light
 // cones); `cones` / `cones_count` (device, nullable) walk only listed cones.
 int visibility_impl(cc_context* ctx, const cc_scene* scene, const float* receivers, uint64_t npoints,

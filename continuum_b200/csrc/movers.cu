@@ -346,8 +346,7 @@ int cc_scene_move(cc_scene* s, const cc_instance* placements, uint32_t n, float*
   };
   if ((rc = put_nodes(0, 3))) return rc;
   if (t.nodes && (rc = put_nodes(t.first_node, t.nodes))) return rc;
-  CC_CUDA(cudaMemcpy(s->items + t.first_item, &f.items[t.first_item], t.objects.size() * 4, cudaMemcpyHostToDevice),
-          "move items");
+  CC_CUDA(copy_in(s->items + t.first_item, &f.items[t.first_item], t.objects.size() * 4), "move items");
   return CC_OK;
 }
 
