@@ -328,7 +328,7 @@ int cc_context_create(int device, cc_context** out) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->copied, cudaEventDisableTiming);
   float disk[64];
   disk_table(disk);
-  if (e == cudaSuccess) e = cc::upload_disk_table(disk);
+  if (e == cudaSuccess) e = cc::device_tables(disk);
   if (e == cudaSuccess) e = ctx->counters.reserve(cc::kCounterWords * sizeof(uint32_t));
   ctx->marks.assign(3 * cc_context::kTimingRing, nullptr);
   for (auto& ev : ctx->marks)

@@ -262,7 +262,9 @@ static_assert(kStaticMaxCones <= kSplitChunk, "a static call is one split chunk"
 // call per device looks it up; later calls return the cached address.
 cudaError_t static_scratch(int device, void** ptr);
 
-cudaError_t upload_disk_table(const float* table64);
+// The tables every context's kernels read (each unit's copy of the disk
+// table, the sky faces), written once on the current device.
+cudaError_t device_tables(const float* disk64);
 // The prefiltering unit's copy of the table, and its plain passes (packet
 // pass with 32-bit cells, or solo pass with 64-bit ones when `wide`).
 cudaError_t upload_disk_table_splat(const float* table64);

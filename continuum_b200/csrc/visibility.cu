@@ -27,20 +27,34 @@
 // stopped early (capped, or every bin full), is listed and walked again
 // alone by a second launch, so every cone's result is the one its own walk
 // gives (the reference's walk without packets, as its view-cache bakes run).
+#include <mutex>
+
 #include "visibility_kernel.cuh"
 
 namespace cc {
 
 // ---- host-side launchers --------------------------------------------------------
 
-cudaError_t upload_disk_table(const float* table64) {
-  cudaError_t e = cudaMemcpyToSymbol(c_disk, table64, kBins * sizeof(float));
-  if (e == cudaSuccess) e = upload_disk_table_split(table64);  // the integrating unit's copy
-  if (e == cudaSuccess) e = upload_disk_table_splat(table64);  // the prefiltering unit's copy
+// Whether this device's tables are written: on the device, so that it is
+// right again in a new primary context. Other contexts' kernels may be reading
+// the tables, so a later context leaves them alone.
+static __device__ uint32_t g_tables_written;
+
+cudaError_t device_tables(const float* disk64) {
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
+  uint32_t written = 0;
+  cudaError_t e = cudaMemcpyFromSymbol(&written, g_tables_written, sizeof written);
+  if (e != cudaSuccess || written) return e;
+  e = cudaMemcpyToSymbol(c_disk, disk64, kBins * sizeof(float));
+  if (e == cudaSuccess) e = upload_disk_table_split(disk64);  // the integrating unit's copy
+  if (e == cudaSuccess) e = upload_disk_table_splat(disk64);  // the prefiltering unit's copy
   if (e != cudaSuccess) return e;
   sky_table_kernel<<<6, 160>>>();
   e = cudaGetLastError();
   if (e == cudaSuccess) e = make_sky_table_splat();
+  written = 1u;
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_tables_written, &written, sizeof written);
   return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
 }
 

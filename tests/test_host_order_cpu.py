@@ -130,3 +130,15 @@ def test_no_kernel_runs_beside_a_copy_of_its_inputs(fake_library, call):
                                           "\nprint('UNORDERED', fake.fake_unordered().decode())\n")
     assert int(out.split("LAUNCHES", 1)[1].split()[0]) > 0
     assert out.split("UNORDERED", 1)[1].strip() == ""
+
+
+def test_a_device_gets_its_tables_once(fake_library):
+    """The tables that every context's kernels read are not written again when
+    another context is created, as those kernels may be running."""
+    out = run(fake_library, """
+made = fake.fake_launches(b"sky_table")
+other = MaskConeKernel(0)
+print(made, fake.fake_launches(b"sky_table"), fake.fake_unordered().decode())
+""")
+    made, after = map(int, out.split())
+    assert made == after == 2  # one copy in each unit that walks sky cones
