@@ -990,7 +990,16 @@ int cc_irradiance(cc_context* ctx, const float* receivers6, uint64_t npoints, co
   // Inputs and the output on the device, then `runs` timed executions; in the
   // context's buffers, as one call at a time runs on a context, and copied in
   // its stream, ahead of the kernels that read them.
-  auto cleanup = [&] { cc_scene_destroy(scene); };
+  // A call that grows one of them past kKept (131,072 receivers, whose walk
+  // takes milliseconds) gives it back, so the context does not hold the
+  // largest call's inputs until it is destroyed.
+  constexpr size_t kKept = size_t(4) << 20;
+  const size_t had_rec = ctx->receivers.size, had_out = ctx->irradiance.size;
+  auto cleanup = [&] {
+    cc_scene_destroy(scene);
+    ctx->receivers.give_back(had_rec, kKept);
+    ctx->irradiance.give_back(had_out, kKept);
+  };
   cudaError_t e = ctx->receivers.reserve(std::max<uint64_t>(npoints, 1) * 32);
   if (e == cudaSuccess) e = ctx->lights.reserve(64);
   if (e == cudaSuccess) e = ctx->irradiance.reserve(std::max<uint64_t>(npoints, 1) * 4);

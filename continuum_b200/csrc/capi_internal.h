@@ -38,6 +38,10 @@ struct DevBuf {
     if (e == cudaSuccess) size = want;
     return e;
   }
+  // Released if it grew past `most` bytes from the `had` it held before.
+  void give_back(size_t had, size_t most) {
+    if (size > had && size > most) release();
+  }
   void release() {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;

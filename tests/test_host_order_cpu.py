@@ -142,3 +142,25 @@ print(made, fake.fake_launches(b"sky_table"), fake.fake_unordered().decode())
 """)
     made, after = map(int, out.split())
     assert made == after == 2  # one copy in each unit that walks sky cones
+
+
+def test_a_large_drop_in_call_keeps_no_inputs(fake_library):
+    """cc_irradiance borrows the context's buffers, and gives back what a large
+    call made them grow by; and a closed context and batch keep nothing."""
+    out = run(fake_library, """
+from continuum_b200.kernel import RectLight
+light = RectLight((-1.0, 6.0, -1.0), (2.0, 0.0, 0.0), (0.0, 0.0, 2.0), True)
+n = 1 << 20
+r6 = np.zeros((n, 6), np.float32)
+r8 = np.zeros((n, 8), np.float32)
+scene = kernel.scene(w.meshes)
+o = {"irradiance": np.zeros(n, np.float32)}
+kernel.visibility_device(scene, r8.ctypes.data, n, lights.ctypes.data, 1, pointers(o))  # the walk's own scratch
+scene.close()
+kernel.irradiance(r6[:64], light, w.meshes)
+before = fake.fake_live_bytes()
+kernel.irradiance(r6, light, w.meshes)
+print(before, fake.fake_live_bytes())
+""")
+    before, after = map(int, out.split())
+    assert after <= before
