@@ -309,7 +309,9 @@ int cc_batch_destroy(cc_batch* b) {
   cudaSetDevice(b->ctx->device);
   if (b->submitted && b->done) cudaEventSynchronize(b->done);
   drop_graph(b);
-  for (DevBuf* d : {&b->job_table, &b->redo, &b->order, &b->sort_scratch, &b->counters, &b->records, &b->masks})
+  for (DevBuf* d : {&b->job_table, &b->redo, &b->order, &b->sort_scratch, &b->counters, &b->records, &b->masks,
+                    &b->upd_perm, &b->upd_flags, &b->upd_list, &b->upd_count, &b->upd_temp, &b->splat_table,
+                    &b->splat_redo, &b->splat_order, &b->splat_sort_scratch})
     d->release();
   if (b->status) cudaFreeHost(b->status);
   if (b->done) cudaEventDestroy(b->done);

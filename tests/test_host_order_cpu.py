@@ -164,3 +164,27 @@ print(before, fake.fake_live_bytes())
 """)
     before, after = map(int, out.split())
     assert after - before <= 2 * (4 << 20)  # two buffers of at most 4 MB
+
+
+def test_closed_contexts_and_batches_keep_nothing(fake_library):
+    out = run(fake_library, """
+empty = fake.fake_live_bytes()
+k = MaskConeKernel(0)
+scene = k.scene(w.meshes)
+k.visibility(scene, rec, lights, outputs=("full", "any", "partial", "irradiance", "fraction", "work"))
+k.sky_visibility(scene, rec, outputs=("full", "fraction"))
+b = Batch(k)
+keep = [outputs() for _ in range(3)]
+stale = np.ones(P * L, np.uint8)
+b.add(scene, rec.ctypes.data, P, lights.ctypes.data, L, pointers(keep[0]))
+b.add(scene, rec.ctypes.data, P, lights.ctypes.data, L, pointers(keep[1]), prefilter=1.0)
+b.add_update(scene, rec.ctypes.data, P, lights.ctypes.data, L, stale.ctypes.data, pointers(keep[2]))
+b.submit(Batch.options(flags=0))
+b.wait()
+b.close()
+scene.close()
+k.close()
+print(empty, fake.fake_live_bytes())
+""")
+    empty, after = map(int, out.split())
+    assert after == empty
