@@ -90,7 +90,13 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
   float v = min_nan(min_nan(fdot(t.nu0, m, fdot_abs(t.nu0, e, 0.0f)), fdot(t.nu1, m, fdot_abs(t.nu1, e, 0.0f))),
                     min_nan(fdot(t.nv0, m, fdot_abs(t.nv0, e, 0.0f)), fdot(t.nv1, m, fdot_abs(t.nv1, e, 0.0f))));
   float n = fm + fe - 2.0f * kNear;
-  if constexpr (kHorizon) n = min_nan(n, fdot(horizon, m, fdot_abs(horizon, e, 0.0f)));
+  // A horizon of zero culls nothing: left out, as its value, zero, would leave
+  // every box that touches to the exact form.
+  if constexpr (kHorizon) {
+    const float h = fdot(horizon, m, fdot_abs(horizon, e, 0.0f));
+    const bool none = horizon.x == 0.0f && horizon.y == 0.0f && horizon.z == 0.0f;
+    n = none ? n : min_nan(n, h);
+  }
   const float f = t.far_rel - fm + fe;
   const float s_far = 2.0f * s_world + kBoxSlack * fabsf(c.far_offset);
   // The bounding cone: axis . d >= bcos sqrt(d.d - r r) - bsin r once outside

@@ -17,6 +17,7 @@ HARNESS = r"""
 #include <cmath>
 #include <cstdio>
 #include <random>
+#include <string>
 #define __device__
 #define __forceinline__ inline
 #define __fmaf_rn fmaf
@@ -44,10 +45,11 @@ static float rsqrt_approx(float x) { return (float)(1.0 / std::sqrt((double)x)) 
 using namespace cc;
 int main(int, char** argv) {
   std::mt19937_64 g(atoi(argv[1]));
+  const std::string form = argv[2];
   auto u = [&] { return (double)(g() >> 11) / 9007199254740992.0; };
   auto U = [&](double a, double b) { return (float)(a + (b - a) * u()); };
   auto L = [&](double a, double b) { return (float)std::exp(std::log(a) + (std::log(b) - std::log(a)) * u()); };
-  long asked = 0, open = 0, wrong = 0;
+  long asked = 0, open = 0, wrong = 0, touching = 0, touching_open = 0;
   for (long it = 0; it < 60000; ++it) {
     const float world = L(0.5, 3000);
     Cone c{};
@@ -75,7 +77,9 @@ int main(int, char** argv) {
     for (int k = 0; k < 4; ++k) ch = fminf(ch, dot(c.baxis, normalize(direction(c, float(k & 1), float(k >> 1)))));
     c.bcos = fminf(fmaxf(ch - 1e-5f, -1.f), 1.f);
     c.bsin = sqrtf(fmaxf(1.f - c.bcos * c.bcos, 0.f));
-    const f3 hz = normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)));
+    f3 hz = normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)));
+    if (form == "no horizon") hz = mk(0, 0, 0);
+    if (form == "any normal") hz = hz * L(1e-4, 1e4);
     if (it % 5003 == 1) c.right.x = NAN;
     if (it % 5003 == 2) c.baxis.y = NAN;
     if (it % 5003 == 3) c.apex.z = INFINITY;
@@ -95,30 +99,51 @@ int main(int, char** argv) {
         lo = mk(fminf(p.x, q.x), fminf(p.y, q.y), fminf(p.z, q.z));
         hi = mk(fmaxf(p.x, q.x), fmaxf(p.y, q.y), fmaxf(p.z, q.z));
       }
+      if (form == "any normal" && k % 3 == 1) {  // the corner farthest along the normal on the horizon
+        const f3 top = mk(hz.x > 0 ? hi.x : lo.x, hz.y > 0 ? hi.y : lo.y, hz.z > 0 ? hi.z : lo.z) - c.apex;
+        const f3 down = hz * (dot(hz, top) / dot(hz, hz));
+        lo = lo - down;
+        hi = hi - down;
+      }
       if (it % 5003 == 4) hi.x = INFINITY;
       for (int h = 0; h < 2; ++h) {
         const bool exact = h ? may_touch_box<true>(c, lo, hi, hz) : may_touch_box<false>(c, lo, hi, hz);
         const int v = h ? box_verdict<true>(c, t, lo, hi, hz) : box_verdict<false>(c, t, lo, hi, hz);
         ++asked;
+        if (exact) ++touching;
+        if (exact && v == 2) ++touching_open;
         if (v == 2) ++open;
         else if ((v == 1) != exact) ++wrong;
       }
     }
   }
-  std::printf("%ld %ld %ld\n", asked, open, wrong);
+  std::printf("%ld %ld %ld %ld %ld\n", asked, open, wrong, touching, touching_open);
 }
 """
 
 
-@pytest.mark.parametrize("seed", [1, 2])
-def test_box_verdict_never_contradicts_the_exact_test(tmp_path, seed):
-    src = tmp_path / "box.cpp"
-    src.write_text(HARNESS)
-    exe = tmp_path / "box"
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("box")
+    (folder / "box.cpp").write_text(HARNESS)
+    exe = folder / "box"
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-Wno-unknown-pragmas", "-I",
-                    str(ROOT / "continuum_b200" / "csrc"), "-o", str(exe), str(src)], check=True)
-    asked, left, wrong = map(int, subprocess.run([str(exe), str(seed)], check=True, capture_output=True,
-                                                 text=True).stdout.split())
+                    str(ROOT / "continuum_b200" / "csrc"), "-o", str(exe), str(folder / "box.cpp")], check=True)
+
+    def run(seed, form):
+        out = subprocess.run([str(exe), str(seed), form], check=True, capture_output=True, text=True).stdout
+        return map(int, out.split())
+
+    return run
+
+
+@pytest.mark.parametrize("form", ["unit", "no horizon"])
+@pytest.mark.parametrize("seed", [1, 2])
+def test_box_verdict_never_contradicts_the_exact_test(harness, seed, form):
+    """`no horizon`: horizons of zero, which cull nothing (CC_SKY_NO_HORIZON_CULL)."""
+    asked, left, wrong, touching, touching_left = harness(seed, form)
     assert wrong == 0
-    # A sixth of the boxes are put on a plane; most others are decided.
+    # A sixth of the boxes are put on a plane; most others are decided, and of
+    # those that touch as many.
     assert left < 0.25 * asked
+    assert touching_left < 0.5 * touching
