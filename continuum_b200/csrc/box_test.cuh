@@ -90,12 +90,15 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
   float v = min_nan(min_nan(fdot(t.nu0, m, fdot_abs(t.nu0, e, 0.0f)), fdot(t.nu1, m, fdot_abs(t.nu1, e, 0.0f))),
                     min_nan(fdot(t.nv0, m, fdot_abs(t.nv0, e, 0.0f)), fdot(t.nv1, m, fdot_abs(t.nv1, e, 0.0f))));
   float n = fm + fe - 2.0f * kNear;
-  // A horizon of zero culls nothing: left out, as its value, zero, would leave
-  // every box that touches to the exact form.
+  // The horizon is the caller's normal, of any length: its slack has its size.
+  // One of zero culls nothing: left out, as its value, zero, would leave every
+  // box that touches to the exact form.
   if constexpr (kHorizon) {
-    const float h = fdot(horizon, m, fdot_abs(horizon, e, 0.0f));
-    const bool none = horizon.x == 0.0f && horizon.y == 0.0f && horizon.z == 0.0f;
-    n = none ? n : min_nan(n, h);
+    const float size = fabsf(horizon.x) + fabsf(horizon.y) + fabsf(horizon.z);
+    const float h = fdot(horizon, m, fdot_abs(horizon, e, 0.0f)), s_h = __fmaf_rn(s_near, size, 1e-36f);
+    // The near plane's verdict stands for both: below both slacks cannot touch,
+    // above both passes, else (not-a-numbers among them) open.
+    n = size == 0.0f || h >= s_h ? n : (h < -s_h ? -INFINITY : min_nan(n, 0.0f));
   }
   const float f = t.far_rel - fm + fe;
   const float s_far = 2.0f * s_world + kBoxSlack * fabsf(c.far_offset);

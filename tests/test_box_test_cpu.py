@@ -137,10 +137,11 @@ def harness(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("form", ["unit", "no horizon"])
+@pytest.mark.parametrize("form", ["unit", "no horizon", "any normal"])
 @pytest.mark.parametrize("seed", [1, 2])
 def test_box_verdict_never_contradicts_the_exact_test(harness, seed, form):
-    """`no horizon`: horizons of zero, which cull nothing (CC_SKY_NO_HORIZON_CULL)."""
+    """`no horizon`: horizons of zero, which cull nothing (CC_SKY_NO_HORIZON_CULL);
+    `any normal`: horizons of any length, and boxes with a corner on theirs."""
     asked, left, wrong, touching, touching_left = harness(seed, form)
     assert wrong == 0
     # A sixth of the boxes are put on a plane; most others are decided, and of
