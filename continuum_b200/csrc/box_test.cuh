@@ -82,7 +82,9 @@ __device__ __forceinline__ BoxTest box_test(const Cone& c) {
 template <bool kHorizon>
 __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 lo, f3 hi, f3 horizon) {
   const f3 a = lo - c.apex, b = hi - c.apex;
-  const f3 m = a + b, e = b - a;  // doubled centre (from the apex) and half extents
+  // Doubled centre (from the apex) and half extents; an uploaded box's corners
+  // may be swapped, which the exact form does not see.
+  const f3 m = a + b, e = mk(fabsf(b.x - a.x), fabsf(b.y - a.y), fabsf(b.z - a.z));
   const float reach = (fabsf(m.x) + e.x) + (fabsf(m.y) + e.y) + (fabsf(m.z) + e.z);
   const float s_near = kBoxSlack * reach, s_side = s_near * t.side;
   const float s_world = __fmaf_rn(kBoxSlack, t.world, s_near);  // half the doubled sums' world coordinates

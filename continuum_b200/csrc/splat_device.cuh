@@ -163,7 +163,7 @@ __device__ __forceinline__ int quick_node_test(const Cone& c, const BoxTest& t, 
   const int v = box_verdict<kHorizon>(c, t, lo, hi, horizon);
   if (v != 1) return v == 0 ? 0 : 4;
   const f3 a = lo - c.apex, b = hi - c.apex;
-  const f3 m = a + b, e = b - a;
+  const f3 m = a + b, e = mk(fabsf(b.x - a.x), fabsf(b.y - a.y), fabsf(b.z - a.z));
   const float reach = (fabsf(m.x) + e.x) + (fabsf(m.y) + e.y) + (fabsf(m.z) + e.z);
   const float slack = kBoxSlack * reach;
   const float fm = fdot(c.fwd, m, 0.0f), fe = fdot_abs(c.fwd, e, 0.0f);

@@ -105,6 +105,12 @@ int main(int, char** argv) {
         lo = lo - down;
         hi = hi - down;
       }
+      if (form == "corners swapped") {
+        if (k & 1) std::swap(lo.x, hi.x);
+        if (k & 2) std::swap(lo.y, hi.y);
+        if (k & 4) std::swap(lo.z, hi.z);
+        if (k == 8) lo = mk(3.4e38f, 3.4e38f, 3.4e38f), hi = -lo;  // an empty box as some builders write it
+      }
       if (it % 5003 == 4) hi.x = INFINITY;
       for (int h = 0; h < 2; ++h) {
         const bool exact = h ? may_touch_box<true>(c, lo, hi, hz) : may_touch_box<false>(c, lo, hi, hz);
@@ -137,11 +143,12 @@ def harness(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("form", ["unit", "no horizon", "any normal"])
+@pytest.mark.parametrize("form", ["unit", "no horizon", "any normal", "corners swapped"])
 @pytest.mark.parametrize("seed", [1, 2])
 def test_box_verdict_never_contradicts_the_exact_test(harness, seed, form):
     """`no horizon`: horizons of zero, which cull nothing (CC_SKY_NO_HORIZON_CULL);
-    `any normal`: horizons of any length, and boxes with a corner on theirs."""
+    `any normal`: horizons of any length, and boxes with a corner on theirs;
+    `corners swapped`: boxes whose low corner is the higher along some axes."""
     asked, left, wrong, touching, touching_left = harness(seed, form)
     assert wrong == 0
     # A sixth of the boxes are put on a plane; most others are decided, and of
