@@ -47,15 +47,17 @@ __device__ __forceinline__ bool may_touch_box(const Cone& c, f3 lo, f3 hi, f3 ho
 // extents, a quarter of the work. Both are f32 evaluations of one real
 // number with errors below 16 units in the last place of the terms they sum
 // (coordinates from the apex, of size `reach`, times 1 + the window's largest
-// side; for the far plane and the bounding cone, world coordinates), so a
-// value farther from zero than 33 of them decides as the exact form would, and
-// any other (not-a-numbers among them) leaves the question to it. All sums
+// side; for the far plane and the bounding cone, world coordinates; all times
+// the axes' largest component, where an object's matrix made it exceed 1), so
+// a value farther from zero than 33 of them decides as the exact form would,
+// and any other (not-a-numbers among them) leaves the question to it. All sums
 // here are doubled: centre x 2 and the whole extents are one subtraction each.
 constexpr float kBoxSlack = 2e-6f;  // 33 x 2^-24
 struct BoxTest {
   f3 nu0, nu1, nv0, nv1;  // the window's planes: right - u0 fwd, u1 fwd - right, up - v0 fwd, v1 fwd - up
   float side;             // 1 + the window's largest side
-  float world;            // the world coordinates' size at the apex
+  float world;            // the world coordinates' size at the apex, times `axes`
+  float axes;             // 1, or the axes' largest component
   float far_rel;          // the far plane's distance along fwd from the apex, doubled
 };
 __device__ __forceinline__ f3 fma3(f3 a, float s, f3 b) {
@@ -67,6 +69,10 @@ __device__ __forceinline__ float fdot(f3 a, f3 b, float s) {
 __device__ __forceinline__ float fdot_abs(f3 a, f3 h, float s) {  // |a| . h + s
   return __fmaf_rn(fabsf(a.x), h.x, __fmaf_rn(fabsf(a.y), h.y, __fmaf_rn(fabsf(a.z), h.z, s)));
 }
+// kPlaced: the cone may be in the space of a placed object, whose matrix need
+// not be a rotation (cc_scene_move and cc_scene_upload take any); else its axes
+// are unit vectors.
+template <bool kPlaced>
 __device__ __forceinline__ BoxTest box_test(const Cone& c) {
   BoxTest t;
   t.nu0 = fma3(c.fwd, -c.u0, c.right);
@@ -74,7 +80,12 @@ __device__ __forceinline__ BoxTest box_test(const Cone& c) {
   t.nv0 = fma3(c.fwd, -c.v0, c.up);
   t.nv1 = fma3(c.fwd, c.v1, -c.up);
   t.side = 1.0f + fmaxf(fmaxf(fabsf(c.u0), fabsf(c.u1)), fmaxf(fabsf(c.v0), fabsf(c.v1)));
-  t.world = fabsf(c.apex.x) + fabsf(c.apex.y) + fabsf(c.apex.z);
+  t.axes = 1.0f;
+  if constexpr (kPlaced) {
+    auto size = [](f3 a) { return fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)); };
+    t.axes = fmaxf(fmaxf(fmaxf(size(c.right), size(c.up)), fmaxf(size(c.fwd), size(c.baxis))), 1.0f);
+  }
+  t.world = t.axes * (fabsf(c.apex.x) + fabsf(c.apex.y) + fabsf(c.apex.z));
   t.far_rel = 2.0f * (c.far_offset - fdot(c.fwd, c.apex, 0.0f));
   return t;
 }
@@ -86,7 +97,7 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
   // may be swapped, which the exact form does not see.
   const f3 m = a + b, e = mk(fabsf(b.x - a.x), fabsf(b.y - a.y), fabsf(b.z - a.z));
   const float reach = (fabsf(m.x) + e.x) + (fabsf(m.y) + e.y) + (fabsf(m.z) + e.z);
-  const float s_near = kBoxSlack * reach, s_side = s_near * t.side;
+  const float s_near = kBoxSlack * t.axes * reach, s_side = s_near * t.side;
   const float s_world = __fmaf_rn(kBoxSlack, t.world, s_near);  // half the doubled sums' world coordinates
   const float fm = fdot(c.fwd, m, 0.0f), fe = fdot_abs(c.fwd, e, 0.0f);
   float v = min_nan(min_nan(fdot(t.nu0, m, fdot_abs(t.nu0, e, 0.0f)), fdot(t.nu1, m, fdot_abs(t.nu1, e, 0.0f))),
@@ -97,7 +108,7 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
   // box that touches to the exact form.
   if constexpr (kHorizon) {
     const float size = fabsf(horizon.x) + fabsf(horizon.y) + fabsf(horizon.z);
-    const float h = fdot(horizon, m, fdot_abs(horizon, e, 0.0f)), s_h = __fmaf_rn(s_near, size, 1e-36f);
+    const float h = fdot(horizon, m, fdot_abs(horizon, e, 0.0f)), s_h = __fmaf_rn(kBoxSlack * reach, size, 1e-36f);
     // The near plane's verdict stands for both: below both slacks cannot touch,
     // above both passes, else (not-a-numbers among them) open.
     n = size == 0.0f || h >= s_h ? n : (h < -s_h ? -INFINITY : min_nan(n, 0.0f));

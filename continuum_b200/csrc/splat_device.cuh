@@ -165,7 +165,7 @@ __device__ __forceinline__ int quick_node_test(const Cone& c, const BoxTest& t, 
   const f3 a = lo - c.apex, b = hi - c.apex;
   const f3 m = a + b, e = mk(fabsf(b.x - a.x), fabsf(b.y - a.y), fabsf(b.z - a.z));
   const float reach = (fabsf(m.x) + e.x) + (fabsf(m.y) + e.y) + (fabsf(m.z) + e.z);
-  const float slack = kBoxSlack * reach;
+  const float slack = kBoxSlack * t.axes * reach;
   const float fm = fdot(c.fwd, m, 0.0f), fe = fdot_abs(c.fwd, e, 0.0f);
   if (fm - fe < -slack) return 3;
   if (t.far_rel - fm - fe < -(2.0f * __fmaf_rn(kBoxSlack, t.world, slack) + kBoxSlack * fabsf(c.far_offset))) return 3;

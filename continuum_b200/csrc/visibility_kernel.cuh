@@ -558,7 +558,7 @@ __device__ __forceinline__ void add_mesh_flat(const DevScene& s, LaneState<WS>& 
 template <class WS>
 static __device__ __noinline__ bool box_in_table(const WS* ws, int owner, f3 lo, f3 hi) {
   const Cone c = load_cone(ws, owner);
-  return touches_box<WS::kSky>(c, box_test(c), lo, hi, load_horizon(ws, owner));
+  return touches_box<WS::kSky>(c, box_test<WS::kWeighted>(c), lo, hi, load_horizon(ws, owner));
 }
 template <class WS>
 __device__ __forceinline__ int table_slot(int lane) {
@@ -732,7 +732,7 @@ __device__ __forceinline__ void walk_splat_pairs(const DevScene& s, LaneState<WS
         test = splat_in_table(ws, (int)owner, s.blas, s.blas_cov, node, prefilter);
       } else {
         const Cone c = load_cone(ws, (int)owner);
-        test = quick_node_test<WS::kSky>(c, box_test(c), node_lo(a), node_lo(b), load_horizon(ws, (int)owner), prefilter);
+        test = quick_node_test<WS::kSky>(c, box_test<WS::kWeighted>(c), node_lo(a), node_lo(b), load_horizon(ws, (int)owner), prefilter);
         if (kCount) atomicAdd(&ws->visited[owner], 1u);
       }
       const int done = (splat ? 0 : 1) + (test == 3 ? (int)count : 0);
@@ -833,7 +833,7 @@ __device__ __forceinline__ void walk_tree(const DevScene& s, LaneState<WS>& st, 
           bl = __float_as_uint(lb.w);
           ar = __float_as_uint(xa.w);
           br = __float_as_uint(xb.w);
-          const BoxTest test = box_test(c);
+          const BoxTest test = box_test<WS::kWeighted>(c);
   #pragma unroll 1
           for (int ch = 0; ch < 2; ++ch) {
             int v = box_verdict<WS::kSky>(c, test, node_lo(ch ? xa : la), node_lo(ch ? xb : lb), horizon);

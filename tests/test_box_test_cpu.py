@@ -83,7 +83,17 @@ int main(int, char** argv) {
     if (it % 5003 == 1) c.right.x = NAN;
     if (it % 5003 == 2) c.baxis.y = NAN;
     if (it % 5003 == 3) c.apex.z = INFINITY;
-    const BoxTest t = box_test(c);
+    if (form == "any axes") {
+      const float grow = L(1, 1e4);
+      f3 row[3] = {normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1))), normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)))};
+      row[2] = normalize(cross(row[0], row[1]));
+      row[1] = cross(row[2], row[0]);
+      if (it % 3 == 0) row[1] = row[1] * U(0.1, 1);
+      for (f3& r : row) r = r * grow;
+      for (f3* a : {&c.right, &c.up, &c.fwd, &c.baxis}) *a = row[0] * a->x + row[1] * a->y + row[2] * a->z;
+      c.far_offset = dot(c.fwd, c.apex) + dist * dot(c.fwd, c.fwd);
+    }
+    const BoxTest t = form == "any axes" ? box_test<true>(c) : box_test<false>(c);
     for (int k = 0; k < 24; ++k) {
       const float size = L(0.001, world);
       f3 e = mk(L(0.01, 1) * size, L(0.01, 1) * size, L(0.01, 1) * size);
@@ -143,12 +153,13 @@ def harness(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("form", ["unit", "no horizon", "any normal", "corners swapped"])
+@pytest.mark.parametrize("form", ["unit", "no horizon", "any normal", "corners swapped", "any axes"])
 @pytest.mark.parametrize("seed", [1, 2])
 def test_box_verdict_never_contradicts_the_exact_test(harness, seed, form):
     """`no horizon`: horizons of zero, which cull nothing (CC_SKY_NO_HORIZON_CULL);
     `any normal`: horizons of any length, and boxes with a corner on theirs;
-    `corners swapped`: boxes whose low corner is the higher along some axes."""
+    `corners swapped`: boxes whose low corner is the higher along some axes;
+    `any axes`: cones in the space of an object whose matrix is no rotation."""
     asked, left, wrong, touching, touching_left = harness(seed, form)
     assert wrong == 0
     # A sixth of the boxes are put on a plane; most others are decided, and of
