@@ -474,13 +474,21 @@ int cc_batch_tune(cc_batch* b, const cc_batch_options* base, uint32_t reps, cc_b
     return -cuda_fail(e, "tune event");
   }
   if (b->submitted) cudaEventSynchronize(b->done);
+  std::vector<float> times;
   float best_ms = 0.0f;
   int best_i = -1;
   for (size_t i = 0; i < cands.size() && rc == CC_OK; ++i) {
     // The first run of a candidate may also size buffers and upload the job
     // table; the best of `reps` runs is kept.
     float cand_ms = 0.0f;
-    for (uint32_t r = 0; r < reps && rc == CC_OK; ++r) {
+    // Packets hold at most kPacketCones: a size above that is the launch of an
+    // earlier candidate, whose time stands for both.
+    size_t twin = 0;
+    while (twin < i && (cc::packet_cones(cands[twin].points_per_warp) != cc::packet_cones(cands[i].points_per_warp) ||
+                        cands[twin].blocks_per_sm != cands[i].blocks_per_sm || cands[twin].flags != cands[i].flags))
+      ++twin;
+    if (twin < i) cand_ms = times[twin];
+    for (uint32_t r = 0; twin == i && r < reps && rc == CC_OK; ++r) {
       rc = prepare(b, cands[i].points_per_warp);
       if (rc) break;
       cudaEventRecord(t0, stream);
@@ -491,6 +499,7 @@ int cc_batch_tune(cc_batch* b, const cc_batch_options* base, uint32_t reps, cc_b
       if (rc == CC_OK && cudaEventElapsedTime(&ms, t0, t1) == cudaSuccess && (r == 0 || ms < cand_ms)) cand_ms = ms;
     }
     if (rc != CC_OK) break;
+    times.push_back(cand_ms);
     if (ms_out && i < max_candidates) ms_out[i] = cand_ms;
     if (best_i < 0 || cand_ms < best_ms) {
       best_ms = cand_ms;

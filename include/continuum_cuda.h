@@ -210,7 +210,9 @@ typedef struct cc_options {
   float wide_extent;         /* WIDE_EXTENT, mask_cones.wgsl:1048 (8.0) */
   uint32_t light_cone_cap;   /* LIGHT_CONE_CAP, mask_cones.wgsl:1052 (4096) */
   uint32_t wide_cone_cap;    /* WIDE_CONE_CAP, mask_cones.wgsl:1056 (512) */
-  uint32_t points_per_warp;  /* cones walked together per warp: 1..32 (32); results do not depend on it */
+  uint32_t points_per_warp;  /* cones walked together per warp, at most: 1..32 (32). Above 16 it means 16, but for exact
+                                sky cones (32); small calls take fewer. Results do not depend on it (the status bits
+                                that say how a cone was walked, cc_outputs.work, may) */
   uint32_t flags;            /* CC_DEVICE_POINTERS, CC_NO_REDO, CC_KEEP_ORDER, CC_NO_OBJECT_PREFILTER, CC_BACK_FACING */
   float prefilter;           /* prefiltered cones (MaskConeKernel::set_prefilter, lib.rs:1508): a hierarchy node
                                 wholly between the near and far planes projecting to at most this many bins is
@@ -349,12 +351,12 @@ typedef struct cc_batch cc_batch;
 #define CC_BATCH_GRAPH 8u /* replay submissions from a captured CUDA graph (cc_batch_options.flags) */
 
 typedef struct cc_batch_options {
-  uint32_t points_per_warp; /* cones per packet: 1..32 (32) */
+  uint32_t points_per_warp; /* cones per packet, at most: 1..32 (32); above 16 it means 16 */
   uint32_t blocks_per_sm;   /* resident blocks per SM launched: 1..8 (8) */
   uint32_t flags;           /* CC_KEEP_ORDER, CC_NO_REDO, CC_BATCH_GRAPH */
 } cc_batch_options;
 
-/* Defaults: 32 cones per packet, 8 blocks per SM, CC_BATCH_GRAPH. */
+/* Defaults: 32 cones per packet at most (16), 8 blocks per SM, CC_BATCH_GRAPH. */
 CC_API void cc_batch_options_default(cc_batch_options* opt);
 
 CC_API int cc_batch_create(cc_context* ctx, cc_batch** out);
@@ -438,7 +440,7 @@ typedef struct cc_server_options {
   uint32_t max_inflight;     /* launches in flight at once: 1..8 (4) */
   uint32_t max_queue;        /* queued requests before submissions are refused with CC_ERR_BUSY (256) */
   uint64_t max_launch_cones; /* cones one launch takes at most (2M); one larger request runs alone */
-  uint32_t points_per_warp;  /* 1..32 (32) */
+  uint32_t points_per_warp;  /* 1..32 (32); above 16 it means 16 */
   uint32_t blocks_per_sm;    /* 1..8 (8) */
   uint32_t deadline_ns_per_cone; /* admission earliest deadline first, deadline = submission + this per
                                     cone (12: about one B200's rate on a plain scene); 0: arrival order */

@@ -112,6 +112,7 @@ def test_every_tuned_configuration_gives_the_same_results(kernel):
     b = jobs.batch(kernel)
     best, ms = b.tune(reps=1)
     assert len(ms) == 12 and np.all(ms > 0)
+    assert np.array_equal(ms[4:8], ms[8:12])  # 16 and 32 cones per packet are one configuration: measured once
     assert best.points_per_warp in (8, 16, 32) and best.blocks_per_sm in (4, 8)
     assert best.flags & _lib.CC_BATCH_GRAPH
     for opt in (best, Batch.options(1, 1, 0), Batch.options(32, 5, _lib.CC_KEEP_ORDER)):
