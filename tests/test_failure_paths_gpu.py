@@ -141,6 +141,28 @@ def deep_chain_scene(kernel, depth):
     return kernel.scene_from_flat(tris, ranges, blas, blas_items, nodes, items)
 
 
+def test_deep_hierarchy_reports_stack_overflow_for_prefiltering_cones(kernel):
+    """The same chain walked by prefiltering cones: every node reaches around
+    the cones' apexes, so each is descended into."""
+    rec = np.zeros((32, 8), np.float32)
+    rec[:, 0] = np.linspace(-1.0, 1.0, 32)
+    rec[:, 5] = 1.0
+    w = scenes.box_field(grid=4)
+    kernel.prefilter = 1.0
+    try:
+        shallow = deep_chain_scene(kernel, 40)
+        v = kernel.visibility(shallow, rec, w.lights, outputs=KEYS + ("work",))
+        assert not (v.work[..., 3] & _lib.CC_CONE_STACK).any()
+        shallow.close()
+        deep = deep_chain_scene(kernel, 80)
+        with pytest.raises(CCError) as e:
+            kernel.visibility(deep, rec, w.lights, outputs=KEYS)
+        assert e.value.code == _lib.CC_ERR_STACK
+        deep.close()
+    finally:
+        kernel.prefilter = 0.0
+
+
 def test_deep_hierarchy_reports_stack_overflow(kernel):
     rec = np.zeros((32, 8), np.float32)
     rec[:, 0] = np.linspace(-1.0, 1.0, 32)

@@ -39,9 +39,10 @@ def sliced_scene(counts, seed=1):
     return meshes, lights, np.concatenate([rec, own]).astype(np.float32)
 
 
-def same(kernel, meshes, lights, rec, cap=4096, wide_cap=512, wide_extent=8.0, pw=32):
+def same(kernel, meshes, lights, rec, cap=4096, wide_cap=512, wide_extent=8.0, pw=32, prefilter=0.0):
     osc = OracleScene(meshes)
-    o = osc.visibility(rec, lights, accumulate=1, light_cone_cap=cap, wide_cone_cap=wide_cap, wide_extent=wide_extent)
+    o = osc.visibility(rec, lights, accumulate=1, light_cone_cap=cap, wide_cone_cap=wide_cap, wide_extent=wide_extent,
+                       prefilter=prefilter)
     osc.close()
     scene = kernel.scene(meshes)
     kernel.light_cone_cap, kernel.wide_cone_cap, kernel.wide_extent = cap, wide_cap, wide_extent
@@ -112,3 +113,89 @@ def test_walk_order_over_any_bounds(kernel, squeeze):
     scene.close()
     for k in ("full", "any", "irradiance", "fraction"):
         assert np.array_equal(getattr(a, k), getattr(b, k), equal_nan=k in ("irradiance", "fraction")), k
+
+
+def flat_copy(kernel, meshes, flip=False):
+    """The scene of `meshes` uploaded as flat arrays; `flip`: with the corners
+    of its hierarchies' boxes swapped along some axes."""
+    built = kernel.scene(meshes)
+    a = built.arrays()
+    built.close()
+    counts = [len(m) for m in meshes]
+    tris = np.zeros((sum(counts), 3, 4), np.float32)
+    tris[:, :, 0:3] = np.concatenate(meshes)
+    blas, nodes = a["blas"].copy(), a["nodes"].copy()
+    if flip:
+        rng = np.random.default_rng(7)
+        for n in (blas, nodes):
+            swap = rng.random((len(n), 3)) < 0.5
+            lo, hi = n["lo"][:, :3].copy(), n["hi"][:, :3].copy()
+            n["lo"][:, :3], n["hi"][:, :3] = np.where(swap, hi, lo), np.where(swap, lo, hi)
+    return kernel.scene_from_flat(tris, a["ranges"], blas, a["blas_items"], nodes, a["items"])
+
+
+def test_swapped_box_corners_change_no_result(kernel):
+    meshes, lights, rec = sliced_scene([1280, 300])
+    out = []
+    for flip in (False, True):
+        scene = flat_copy(kernel, meshes, flip)
+        out.append(kernel.visibility(scene, rec, lights))
+        scene.close()
+    for k in ("full", "any", "irradiance", "fraction"):
+        assert np.array_equal(getattr(out[0], k), getattr(out[1], k)), k
+
+
+def fullest_stack(cones, depth, room):
+    """The most pairs waiting in a walk of a complete tree, every node touched:
+    32 at a time, or one once `room` are waiting."""
+    stack, most = [0] * cones, 0
+    while stack:
+        n = min(len(stack), 32, max(room - len(stack), 1))
+        taken = stack[-n:]
+        del stack[-n:]
+        for d in taken:
+            if d + 1 < depth:
+                stack += [d + 1, d + 1]
+        most = max(most, len(stack))
+    return most
+
+
+@pytest.mark.parametrize("cap", [1 << 20, 4096])
+@pytest.mark.parametrize("prefilter", [0.0, 1e-3])
+def test_full_pair_stack(kernel, prefilter, cap):
+    """A sheet of 8,192 triangles wholly inside every cone: the pairs waiting
+    fill the stack to where they are taken one by one (192 of 256; prefiltering
+    cones 256 of 384), and with the smaller cap the cones are walked again in
+    order from there."""
+    n = 64
+    g = np.linspace(-0.4, 0.4, n + 1)
+    x, z = (a.astype(np.float32) for a in np.meshgrid(g, g, indexing="ij"))
+    at = np.stack([x, np.full_like(x, 2.0), z], axis=-1)
+    p00, p10, p01, p11 = at[:-1, :-1], at[1:, :-1], at[:-1, 1:], at[1:, 1:]
+    sheet = np.concatenate([np.stack([p00, p10, p11], axis=2).reshape(-1, 3, 3),
+                            np.stack([p00, p11, p01], axis=2).reshape(-1, 3, 3)])
+    depth = 10  # 1,024 leaves of eight triangles, or fewer in each
+    assert fullest_stack(16, depth, 192) > 192 and fullest_stack(16, depth, 256) > 256
+    lights = np.stack([light_gpu(Light.rect(RectLight((-2.0, 4.0, -2.0), (4.0, 0.0, 0.0), (0.0, 0.0, 4.0), True)))])
+    rec = np.zeros((64, 8), np.float32)
+    rec[:, 0], rec[:, 2] = np.tile(np.linspace(-0.1, 0.1, 8), 8), np.repeat(np.linspace(-0.1, 0.1, 8), 8)
+    rec[:, 5] = 1.0
+    meshes = [np.ascontiguousarray(sheet, np.float32)]
+    kernel.prefilter = prefilter
+    try:
+        work = same(kernel, meshes, lights, rec, cap=cap, prefilter=prefilter)
+    finally:
+        kernel.prefilter = 0.0
+    assert (work[:, 3] & 1).all() == (cap == 4096)
+
+
+@pytest.mark.parametrize("cap,wide_cap", [(9, 9), (40, 20)])
+@pytest.mark.parametrize("prefilter", [0.25, 1.0])
+def test_prefiltered_caps_inside_a_mesh(kernel, cap, wide_cap, prefilter):
+    kernel.prefilter = prefilter
+    try:
+        work = same(kernel, *sliced_scene([1280, 640], seed=3), cap=cap, wide_cap=wide_cap, wide_extent=0.5,
+                    prefilter=prefilter)
+    finally:
+        kernel.prefilter = 0.0
+    assert (work[:, 3] & 1).any()
