@@ -1028,6 +1028,49 @@ def reference_arm(args, rank: int) -> None:
     print(json.dumps(line), flush=True)
 
 
+def headline(record: dict) -> dict:
+    """The one line on standard output: the record's own figures, and of each
+    leg its rates and times. The whole record, with every rate's, frame's and
+    sample's figures, is 28 KB, more than a reader of the last few kilobytes of
+    the output gets whole; it goes to standard error."""
+    legs = {"small": ("value", "unit", "ms_per_step"),
+            "batched": ("value", "unit", "ms_per_step", "speedup_vs_plain_per_job"),
+            "sky": (), "instanced": (), "bake": (), "served": (), "accuracy": ()}
+    line = {k: v for k, v in record.items() if k not in legs}
+    for leg, keys in legs.items():
+        if record.get(leg) is not None:
+            line[leg] = {k: record[leg].get(k) for k in keys}
+
+    def pick(leg: str, part: str, *keys: str) -> None:
+        if leg in line and record[leg].get(part) is not None:
+            line[leg][part] = {k: record[leg][part].get(k) for k in keys}
+
+    pick("small", "e2e", "value", "unit", "ms_per_step")
+    pick("batched", "plain_per_job", "value", "ms_per_step")
+    pick("sky", "exact", "value", "unit", "ms")
+    pick("sky", "prefiltered", "value", "unit", "ms")
+    pick("instanced", "full_solve", "value", "unit", "ms")
+    pick("instanced", "update", "ms_per_frame", "cones_per_s_served")
+    pick("bake", "fixed_budget", "value", "unit", "frames_to_warm")
+    if "served" in line:
+        keys = ("rate_req_s", "completed", "refused", "p50_ms", "p99_ms", "queries_per_s")
+        line["served"]["rates"] = [{k: r.get(k) for k in keys} for r in record["served"].get("rates", ())]
+    if "accuracy" in line:
+        parts = {}
+        for name, part in record["accuracy"].items():
+            nested = [p for p in part.values() if isinstance(p, dict) and "meets_bar" in p]
+            parts[name] = {"word_agreement": min(p["word_agreement"] for p in nested or [part]),
+                           "meets_bar": all(p["meets_bar"] for p in nested or [part])}
+        line["accuracy"] = parts
+    if record.get("cpu_baseline") is not None:
+        line["cpu_baseline"] = {k: v for k, v in record["cpu_baseline"].items() if not isinstance(v, dict)}
+        for leg in ("threads_1", "threads_all"):
+            path = record["cpu_baseline"].get("cpu_path", {}).get(leg)
+            if path is not None:
+                line["cpu_baseline"]["cpu_path_" + leg] = path["value"]
+    return line
+
+
 def cuda_arm(args, rank: int, world: int, local_rank: int) -> None:
     import torch
 
@@ -1235,7 +1278,8 @@ def cuda_arm(args, rank: int, world: int, local_rank: int) -> None:
                 w, oscene, [i for i in range(L) if w.lights[i][3] < 1.5], max_points=args.cpu_path_points)
     if oscene is not None:
         oscene.close()
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(headline(line)), flush=True)
     scene.close()
     kernel.close()
 

@@ -65,3 +65,31 @@ def test_reference_arm_loads_no_library():
     line = json.loads([l for l in out.stdout.splitlines() if l.startswith("{")][0])
     assert line["impl"] == "reference" and line["unit"] == "cones/s" and line["value"] > 0
     assert line["cpu_path"]["threads_1"]["value"] > 0 and line["cpu_path"]["bvh_build_ms"] > 0
+
+
+def test_the_line_stays_short():
+    """A record as large as the full run's gives a line of a few kilobytes with
+    every figure of the step itself."""
+    import json
+
+    import bench
+
+    accuracy = {"word_agreement": 1.0, "meets_bar": True, "note": "x" * 400}
+    record = {"metric": "m", "value": 1.0, "unit": "cones/s", "ms_per_step": 2.0, "clocks": {"sm_mhz": 1965.0},
+              "e2e": {"value": 3.0, "unit": "cones/s", "h2d_bytes_per_step": 4, "d2h_bytes_per_step": 5},
+              "gpu_launches": 6, "config": {"workload": "w"},
+              "accuracy": {"plain_at_scale": accuracy, "served": accuracy,
+                           "instanced": {"full_solve": accuracy, "after_moves": dict(accuracy, meets_bar=False)}},
+              "small": {"value": 1.0, "unit": "cones/s", "ms_per_step": 1.0, "accuracy": accuracy, "e2e": {"value": 2.0}},
+              "served": {"rates": [dict(rate_req_s=r, p50_ms=1.0, slowest=["x" * 1000] * 3) for r in range(6)]},
+              "instanced": {"full_solve": {"value": 1.0, "ms": 2.0}, "frames": ["x" * 200] * 9},
+              "sky": {"exact": {"value": 1.0, "ms": 2.0, "timing": "t"}},
+              "cpu_baseline": {"value": 1.0, "cores": 16, "cpu_path": {"threads_1": {"value": 7.0, "note": "x" * 900}}}}
+    line = bench.headline(record)
+    for k in ("metric", "value", "unit", "ms_per_step", "clocks", "e2e", "gpu_launches", "config"):
+        assert line[k] == record[k]
+    assert len(json.dumps(record)) > 20_000 and len(json.dumps(line)) < 4_000
+    assert [r["rate_req_s"] for r in line["served"]["rates"]] == list(range(6))
+    assert line["accuracy"]["plain_at_scale"]["meets_bar"] and not line["accuracy"]["instanced"]["meets_bar"]
+    assert line["cpu_baseline"]["cpu_path_threads_1"] == 7.0
+    assert "batched" not in line and line["instanced"]["full_solve"]["ms"] == 2.0
