@@ -1,4 +1,4 @@
-"""The short box test against the exact one, on the host.
+"""The short box and node tests against the exact ones, on the host.
 
 box_test.cuh's box_verdict must never contradict may_touch_box: it answers
 only where f32 rounding cannot change the answer, and leaves the rest to it.
@@ -41,8 +41,21 @@ static f3 to_local(const Cone& c, f3 p) { const f3 d = p - c.apex; return {dot(c
 static float min_nan(float a, float b) { return std::isnan(a) || std::isnan(b) ? NAN : fminf(a, b); }
 static float rsqrt_approx(float x) { return (float)(1.0 / std::sqrt((double)x)) * (1.0f + 2e-7f); }
 #include "box_test.cuh"
+constexpr int kGrid = 8;
+struct float2 { float x, y; };
+struct float4 { float x, y, z, w; };
+static float2 make_float2(float x, float y) { return {x, y}; }
+static float4 make_float4(float x, float y, float z, float w) { return {x, y, z, w}; }
+static float __fdividef(float a, float b) {  // within 2 units in the last place, either way
+  static int n;
+  return a / b * (n++ & 1 ? 1.0f + 2.4e-7f : 1.0f - 2.4e-7f);
+}
+#include "node_test.cuh"
 }  // namespace cc
 using namespace cc;
+"""
+
+BOX_MAIN = r"""
 int main(int, char** argv) {
   std::mt19937_64 g(atoi(argv[1]));
   const std::string form = argv[2];
@@ -137,20 +150,93 @@ int main(int, char** argv) {
 }
 """
 
+NODE_MAIN = r"""
+int main(int, char** argv) {
+  std::mt19937_64 g(atoi(argv[1]));
+  auto u = [&] { return (double)(g() >> 11) / 9007199254740992.0; };
+  auto U = [&](double a, double b) { return (float)(a + (b - a) * u()); };
+  auto L = [&](double a, double b) { return (float)std::exp(std::log(a) + (std::log(b) - std::log(a)) * u()); };
+  long asked = 0, quick = 0, wrong = 0, splats = 0;
+  for (long it = 0; it < 60000; ++it) {
+    const float world = L(0.5, 3000);
+    Cone c{};
+    c.apex = mk(U(-world, world), U(0, world * 0.1), U(-world, world));
+    c.fwd = normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)));
+    c.right = normalize(cross(std::fabs(c.fwd.x) > 0.9f ? mk(0, 1, 0) : mk(1, 0, 0), c.fwd));
+    c.up = cross(c.fwd, c.right);
+    const bool narrow = it % 3 == 0;  // a small light far to the side
+    const float ext = narrow ? L(1e-4, 0.01) : L(0.003, 12);
+    c.u0 = narrow ? U(-40, 40) : U(-3, 3);
+    c.v0 = narrow ? U(-40, 40) : U(-3, 3);
+    c.u1 = c.u0 + ext;
+    c.v1 = c.v0 + ext * U(0.3, 1);
+    const float dist = L(0.01, world * 1.5);
+    c.far_offset = dot(c.fwd, c.apex) + dist * (1 - 1e-5f);
+    c.baxis = normalize(direction(c, 0.5f, 0.5f));
+    float ch = 1;
+    for (int k = 0; k < 4; ++k) ch = fminf(ch, dot(c.baxis, normalize(direction(c, float(k & 1), float(k >> 1)))));
+    c.bcos = fminf(fmaxf(ch - 1e-5f, -1.f), 1.f);
+    c.bsin = sqrtf(fmaxf(1.f - c.bcos * c.bcos, 0.f));
+    const f3 hz = normalize(mk(U(-1, 1), U(-1, 1), U(-1, 1)));
+    const BoxTest t = box_test<false>(c);
+    for (int k = 0; k < 24; ++k) {
+      const float z = L(1e-4, dist * 1.2);
+      const float uu = c.u0 + (c.u1 - c.u0) * U(-0.1, 1.1), vv = c.v0 + (c.v1 - c.v0) * U(-0.1, 1.1);
+      f3 at = c.apex + (c.fwd + c.right * uu + c.up * vv) * z;
+      const float size = ext * z * L(0.01, 30);
+      const f3 e = mk(L(0.01, 1) * size, L(0.01, 1) * size, L(0.01, 1) * size);
+      if (k % 4 == 1) {  // its first or last corner along the cone's axis at a plane
+        const float low = std::fabs(c.fwd.x) * e.x + std::fabs(c.fwd.y) * e.y + std::fabs(c.fwd.z) * e.z;
+        const float planes[3] = {0.0f, kNear, dist * (1 - 1e-5f)};
+        const int p = (k / 4) % 3;
+        at = at + c.fwd * (planes[p] * (1 + U(-1e-6, 1e-6)) + (p == 2 ? -0.5f : 0.5f) * low - dot(c.fwd, at - c.apex));
+      }
+      const f3 lo = at - e * 0.5f, hi = at + e * 0.5f;
+      float2 pts[8];
+      float4 bins{};
+      project_node<false>(c, hz, lo, hi, 3.4e38f, pts, bins);
+      const float width = fmaxf(bins.z - bins.x, bins.w - bins.y);  // of the corners before the first one outside
+      for (int h = 0; h < 4; ++h) {
+        const float prefilter = h < 2 && width > 0 && width < 1e9f ? width * (1 + U(-1, 1) * L(1e-7, 1e-2)) : L(0.1, 8);
+        const int exact = h & 1 ? project_node<true>(c, hz, lo, hi, prefilter, pts, bins)
+                                : project_node<false>(c, hz, lo, hi, prefilter, pts, bins);
+        const int v = h & 1 ? quick_node_test<true>(c, t, lo, hi, hz, prefilter)
+                            : quick_node_test<false>(c, t, lo, hi, hz, prefilter);
+        ++asked;
+        if (exact == 1) ++splats;
+        if (v == 4) continue;
+        ++quick;
+        if (v != exact) ++wrong;
+      }
+    }
+  }
+  std::printf("%ld %ld %ld %ld\n", asked, quick, wrong, splats);
+}
+"""
 
-@pytest.fixture(scope="module")
-def harness(tmp_path_factory):
-    folder = tmp_path_factory.mktemp("box")
-    (folder / "box.cpp").write_text(HARNESS)
-    exe = folder / "box"
+
+def built(tmp_path_factory, name, main):
+    folder = tmp_path_factory.mktemp(name)
+    (folder / "main.cpp").write_text(HARNESS + main)
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-Wno-unknown-pragmas", "-I",
-                    str(ROOT / "continuum_b200" / "csrc"), "-o", str(exe), str(folder / "box.cpp")], check=True)
+                    str(ROOT / "continuum_b200" / "csrc"), "-o", str(folder / name), str(folder / "main.cpp")],
+                   check=True)
 
-    def run(seed, form):
-        out = subprocess.run([str(exe), str(seed), form], check=True, capture_output=True, text=True).stdout
+    def run(*args):
+        out = subprocess.run([str(folder / name), *map(str, args)], check=True, capture_output=True, text=True).stdout
         return map(int, out.split())
 
     return run
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    return built(tmp_path_factory, "box", BOX_MAIN)
+
+
+@pytest.fixture(scope="module")
+def node_harness(tmp_path_factory):
+    return built(tmp_path_factory, "node", NODE_MAIN)
 
 
 @pytest.mark.parametrize("form", ["unit", "no horizon", "any normal", "corners swapped", "any axes"])
@@ -166,3 +252,14 @@ def test_box_verdict_never_contradicts_the_exact_test(harness, seed, form):
     # those that touch as many.
     assert left < 0.25 * asked
     assert touching_left < 0.5 * touching
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_quick_node_test_never_contradicts_the_exact_one(node_harness, seed):
+    """Prefiltering cones at nodes as wide as the prefilter (and a little more
+    or less), with corners at the apex's, the near and the far plane, and in
+    narrow windows far from the axis: where the quick test answers, the exact
+    one agrees; both answers and splats occur."""
+    asked, quick, wrong, splats = node_harness(seed)
+    assert wrong == 0
+    assert quick > 0.4 * asked and splats > 0.05 * asked
