@@ -89,9 +89,25 @@ __device__ __forceinline__ BoxTest box_test(const Cone& c) {
   t.far_rel = 2.0f * (c.far_offset - fdot(c.fwd, c.apex, 0.0f));
   return t;
 }
+// A sky cone's horizon as the tests take it. The caller's normal may have any
+// length, and the plane's error has its size: scaled by a power of two to a
+// largest component in [1/2, 1), which changes no sign of the exact form, it
+// has the slack of the other planes. One of zero (CC_SKY_NO_HORIZON_CULL) culls
+// nothing and gets a value far above the slack, as zero would leave every box
+// that touches to the exact form.
+struct Horizon {
+  f3 normal;
+  float lift;
+};
+__device__ __forceinline__ Horizon scaled_horizon(f3 n) {
+  const float size = fmaxf(fmaxf(fabsf(n.x), fabsf(n.y)), fabsf(n.z));
+  const uint32_t e = __float_as_uint(size) >> 23;  // 2^(e - 127) <= size, but for subnormal sizes
+  const float scale = e < 253u ? __uint_as_float((253u - e) << 23) : 2.9387359e-39f;  // 2^-128
+  return {n * scale, size == 0.0f ? 1e30f : 0.0f};
+}
 // 0: the cone cannot touch the box, 1: it may, 2: ask may_touch_box.
 template <bool kHorizon>
-__device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 lo, f3 hi, f3 horizon) {
+__device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 lo, f3 hi, const Horizon& h) {
   const f3 a = lo - c.apex, b = hi - c.apex;
   // Doubled centre (from the apex) and half extents; an uploaded box's corners
   // may be swapped, which the exact form does not see.
@@ -103,16 +119,7 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
   float v = min_nan(min_nan(fdot(t.nu0, m, fdot_abs(t.nu0, e, 0.0f)), fdot(t.nu1, m, fdot_abs(t.nu1, e, 0.0f))),
                     min_nan(fdot(t.nv0, m, fdot_abs(t.nv0, e, 0.0f)), fdot(t.nv1, m, fdot_abs(t.nv1, e, 0.0f))));
   float n = fm + fe - 2.0f * kNear;
-  // The horizon is the caller's normal, of any length: its slack has its size.
-  // One of zero culls nothing: left out, as its value, zero, would leave every
-  // box that touches to the exact form.
-  if constexpr (kHorizon) {
-    const float size = fabsf(horizon.x) + fabsf(horizon.y) + fabsf(horizon.z);
-    const float h = fdot(horizon, m, fdot_abs(horizon, e, 0.0f)), s_h = __fmaf_rn(kBoxSlack * reach, size, 1e-36f);
-    // The near plane's verdict stands for both: below both slacks cannot touch,
-    // above both passes, else (not-a-numbers among them) open.
-    n = size == 0.0f || h >= s_h ? n : (h < -s_h ? -INFINITY : min_nan(n, 0.0f));
-  }
+  if constexpr (kHorizon) n = min_nan(n, fdot(h.normal, m, fdot_abs(h.normal, e, h.lift)));
   const float f = t.far_rel - fm + fe;
   const float s_far = 2.0f * s_world + kBoxSlack * fabsf(c.far_offset);
   // The bounding cone: axis . d >= bcos sqrt(d.d - r r) - bsin r once outside
@@ -132,8 +139,8 @@ __device__ __forceinline__ int box_verdict(const Cone& c, const BoxTest& t, f3 l
 }
 // may_touch_box's answer.
 template <bool kHorizon>
-__device__ __forceinline__ bool touches_box(const Cone& c, const BoxTest& t, f3 lo, f3 hi, f3 horizon) {
-  int v = box_verdict<kHorizon>(c, t, lo, hi, horizon);
-  if (v == 2) v = may_touch_box<kHorizon>(c, lo, hi, horizon) ? 1 : 0;
+__device__ __forceinline__ bool touches_box(const Cone& c, const BoxTest& t, f3 lo, f3 hi, const Horizon& h) {
+  int v = box_verdict<kHorizon>(c, t, lo, hi, h);
+  if (v == 2) v = may_touch_box<kHorizon>(c, lo, hi, h.normal) ? 1 : 0;
   return v == 1;
 }

@@ -54,9 +54,9 @@ __device__ __forceinline__ int project_node(const Cone& c, f3 horizon, f3 lo, f3
 // projections' distance is a lower bound of that width. Every comparison
 // leaves box_verdict's slack, so the answer is node_cone_test's.
 template <bool kHorizon>
-__device__ __forceinline__ int quick_node_test(const Cone& c, const BoxTest& t, f3 lo, f3 hi, f3 horizon,
+__device__ __forceinline__ int quick_node_test(const Cone& c, const BoxTest& t, f3 lo, f3 hi, const Horizon& h,
                                                float prefilter) {
-  const int v = box_verdict<kHorizon>(c, t, lo, hi, horizon);
+  const int v = box_verdict<kHorizon>(c, t, lo, hi, h);
   if (v != 1) return v == 0 ? 0 : 4;
   const f3 a = lo - c.apex, b = hi - c.apex;
   const f3 m = a + b, e = mk(fabsf(b.x - a.x), fabsf(b.y - a.y), fabsf(b.z - a.z));

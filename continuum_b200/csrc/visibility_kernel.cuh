@@ -72,7 +72,7 @@ struct WarpShared {
   uint32_t queue[kQueueCap];            // (cone, triangle) pairs that passed the cull, waiting to be rasterized
   uint32_t general[kQueueCap];          // pairs that need rasterize's general path, waiting for it
   uint32_t overflow[4];                 // word 0: cones whose 32-bit accumulation overflowed in the current mesh
-  float horizon[Sky ? (3 * kCones + 3 & ~3) : 4];  // sky cones: each cone's horizon, field-major
+  float horizon[Sky ? 4 * kCones : 4];  // sky cones: each cone's horizon (scaled_horizon), field-major
   float cov[SmemCov ? kBins * 32 : 4];  // each cone's 64 coverages, bin-major, lane innermost
   // The placed object being walked (Weighted): its triangles' weight and its
   // transmission (add_mesh_coverage_if's tri_weight / tri_transmit /
@@ -204,16 +204,19 @@ template <class WS>
 __device__ __forceinline__ void store_horizon(WS* ws, f3 h, int lane) {
   if constexpr (WS::kSky) {
     if (WS::kCones < 32 && lane >= WS::kCones) return;
-    ws->horizon[lane] = h.x;
-    ws->horizon[WS::kCones + lane] = h.y;
-    ws->horizon[2 * WS::kCones + lane] = h.z;
+    const Horizon s = scaled_horizon(h);
+    ws->horizon[lane] = s.normal.x;
+    ws->horizon[WS::kCones + lane] = s.normal.y;
+    ws->horizon[2 * WS::kCones + lane] = s.normal.z;
+    ws->horizon[3 * WS::kCones + lane] = s.lift;
   }
 }
 template <class WS>
-__device__ __forceinline__ f3 load_horizon(const WS* ws, int owner) {
+__device__ __forceinline__ Horizon load_horizon(const WS* ws, int owner) {
   if constexpr (WS::kSky)
-    return mk(ws->horizon[owner], ws->horizon[WS::kCones + owner], ws->horizon[2 * WS::kCones + owner]);
-  return mk(0.f, 0.f, 0.f);
+    return {mk(ws->horizon[owner], ws->horizon[WS::kCones + owner], ws->horizon[2 * WS::kCones + owner]),
+            ws->horizon[3 * WS::kCones + owner]};
+  return {mk(0.f, 0.f, 0.f), 0.f};
 }
 
 template <class WS>
@@ -438,7 +441,7 @@ __device__ __noinline__ uint32_t cover_leaf(const float4* __restrict__ tris, WS*
       owner = (int)__fns(owners, 0, r + 1);
       t = t0 + k;
       const Cone c = load_cone(ws, owner);
-      pass = pair_survives<WS::kSky>(tris, c, corners_of(c), load_horizon(ws, owner), t);
+      pass = pair_survives<WS::kSky>(tris, c, corners_of(c), load_horizon(ws, owner).normal, t);
       entry = ((uint32_t)owner << kQueueOwnerShift) | t;
     }
     // The owner's own triangle is not drawn (cover_triangle's cover_skip, :595).
@@ -584,7 +587,7 @@ static __device__ __noinline__ uint32_t cull_leaves(const float4* __restrict__ t
     nt = __float_as_uint(__ldg(&node[1].w));
   }
   const Cone c = load_cone(ws, owner);
-  const f3 horizon = load_horizon(ws, owner);
+  const f3 horizon = load_horizon(ws, owner).normal;
   const Corners w = corners_of(c);
   // The owner's own triangle is not drawn (cover_triangle's cover_skip, :595).
   [[maybe_unused]] uint32_t own = kNoneU;
@@ -618,7 +621,7 @@ static __device__ __noinline__ int splat_in_table(WS* ws, int owner, const float
   const Cone c = load_cone(ws, owner);
   const float4 a = __ldg(&blas[2 * (size_t)node]), b = __ldg(&blas[2 * (size_t)node + 1]);
   LaneAcc<typename WS::Cell, WS::kCones> acc{ws->acc + owner, 68u, 0u, &ws->overflow[0], 1u << owner};
-  const int test = node_cone_test<WS::kSky>(c, load_horizon(ws, owner), acc, cov + kCoverageSamples * (size_t)node,
+  const int test = node_cone_test<WS::kSky>(c, load_horizon(ws, owner).normal, acc, cov + kCoverageSamples * (size_t)node,
                                             node_lo(a), node_lo(b), prefilter);
   note_span(ws, owner, acc);
   return test;
@@ -828,7 +831,7 @@ __device__ __forceinline__ void walk_tree(const DevScene& s, LaneState<WS>& st, 
           const float4* rec = s.blas + 2 * (size_t)left;
           const float4 la = __ldg(rec + 0), lb = __ldg(rec + 1), xa = __ldg(rec + 2), xb = __ldg(rec + 3);
           const Cone c = load_cone(ws, (int)owner);
-          const f3 horizon = load_horizon(ws, (int)owner);
+          const Horizon horizon = load_horizon(ws, (int)owner);
           al = __float_as_uint(la.w);
           bl = __float_as_uint(lb.w);
           ar = __float_as_uint(xa.w);
