@@ -8,7 +8,8 @@ hits of a 1280 x 720 camera: 3,686,400 cones. Synthetic, seeded data.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl cuda|reference]
 
-The CUDA arm prints one JSON line with the device-resident throughput
+The CUDA arm prints one JSON line (and the whole record, with each leg's
+details, to standard error) with the device-resident throughput
 (`value`), the end-to-end throughput through the C ABI with host buffers
 (`e2e`), the dominant kernel's roofline, timed CPU baselines (the oracle's
 FP32 restatement of the reference's GPU path on every host core, and its
@@ -49,10 +50,10 @@ TRI_BYTES = 48   # three vec4 vertices (hierarchy.rs:12-13)
 
 
 # The full plain workload's cones per step, and the DRAM bytes of one
-# packet-pass launch over them as ncu measured them (1.475 GB read + 1.453 GB
-# written, 39.19 ms).
+# packet-pass launch over them as ncu measured them (1.374 GB read + 1.398 GB
+# written, 31.36 ms).
 FULL_CONES = 3_686_400
-PACKET_PASS_DRAM_BYTES = 1_474_594_048 + 1_453_315_584
+PACKET_PASS_DRAM_BYTES = 1_374_164_736 + 1_397_616_384
 
 
 def workload(points: int = 0, caster: str = "library"):

@@ -2,10 +2,10 @@
 //
 // One lane owns one cone. The geometry follows the reference's WGSL light-cone
 // path (crates/continuum-gpu/src/mask_cones.wgsl, cited per function); the
-// per-cone state that the WGSL keeps in private arrays (64 coverages, the
-// 68-cell accumulator) lives here in shared memory, lane-interleaved
-// (cell * 32 + lane), so every access is bank-conflict-free whatever cell
-// each lane touches.
+// 68-cell accumulator that the WGSL keeps in a private array lives here in
+// shared memory, interleaved by cone (cell * a packet's cones + cone), so any
+// lane can add to any cone's cells; the 64 coverages are thread-local, or in
+// shared memory where other lanes integrate them.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

@@ -14,7 +14,8 @@ constexpr int kWarpsPerBlock = 2;
 // so a packet of 16 keeps the lanes as busy as one of 32, with half the shared
 // memory and half the time of the heaviest packet, which ends the pass: 32, 16
 // and 8 cones took 41.3, 40.2 and 45.3 ms on 3.69 M cones over 3.07 M
-// triangles and 10.7, 7.2 and 5.9 ms on 229 k cones. Prefiltering cones too
+// triangles and 10.7, 7.2 and 5.9 ms on 229 k cones, between which 16 is the
+// middle: nothing here takes 8 for the smaller call. Prefiltering cones too
 // (32 and 16 cones: sky 33.6 and 27.0 ms, light 18.6 and 16.3). Exact sky cones
 // keep 32 (4.9 and 5.9 ms): they walk little and integrate a lane each.
 constexpr uint32_t kPacketCones = 16;
@@ -40,7 +41,14 @@ constexpr int kWarpsPerSm = kWarpsPerBlock * kBlocksPerSm;
 // Cones a launch of `cones` walks per packet: at most `most`, halved (down to
 // 2) while the packets would leave resident warps idle: a small call is the
 // time of its heaviest packet. With integrate_slots, host calls of 4,096 cones
-// 468 -> 340 us; 65,536 cones keep packets of 16.
+// 468 -> 340 us; 65,536 cones keep packets of 16. Plain calls only: batches and
+// servers keep their packets, and an update's are those of all its cones. The
+// price is paid by cones that nothing shades, whose packets cost their fixed
+// part: against the build before the tree walk and these rules, 16,384 cones
+// over 40 spheres take 0.16 ms for 0.13 where no sphere shades them, and 0.52
+// for 1.90 where some do. Halving only while one resident wave holds the packets
+// takes 0.14 in the first case, but 0.58 (and 1.00 for 0.72 at 36,000 cones) in
+// the second.
 constexpr uint32_t launch_packet_cones(uint32_t most, uint64_t cones, int sm_count) {
   while (most > 2 && cones / most < (uint64_t)sm_count * kWarpsPerSm) most = (most + 1) / 2;
   return most;

@@ -1,7 +1,8 @@
 // The order in which receivers are walked: Morton order of their positions.
 //
-// A warp walks up to 32 cones together and visits the union of the nodes
-// its cones need, so cones in a warp should see the same geometry. Callers
+// A warp walks up to 32 cones together: one object hierarchy walk visits the
+// union of the nodes its cones need, and their mesh walks share what they load,
+// so cones in a warp should see the same geometry. Callers
 // list receivers in their own order (image rows, texels of many pages); here
 // each receiver gets a Morton code of its position quantized in the scene's
 // bounds, and a device radix sort yields the walk order. Results do

@@ -1,7 +1,8 @@
-// The plain visibility kernel: one warp walks a packet of up to 32 cones
-// (neighbouring points toward one light) through the scene hierarchy
-// together; the lanes share the rasterization of every leaf the packet
-// visits, and each lane integrates its own cone.
+// The plain visibility kernel: one warp walks a packet of up to 16 cones
+// (neighbouring points toward one light; 32 exact sky cones) through the scene
+// hierarchy together; the lanes share the rasterization of every leaf the
+// packet visits. The masks are integrated by a kernel of their own
+// (visibility_split.cu); sky and prefiltering cones by the walk's own warp.
 //
 // What the reference does per invocation (mask_cones.wgsl `main` :1513-1520
 // -> hit_irradiance_rect :2125 -> cone_irradiance_rect :1286) is done here

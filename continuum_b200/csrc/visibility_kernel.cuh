@@ -555,9 +555,8 @@ __device__ __forceinline__ void add_mesh_flat(const DevScene& s, LaneState<WS>& 
 
 // may_touch_box for the table's cone `owner`. Out of line, for the tests that
 // run seldom: the object walk's, the meshes' roots', the in-order walk's and
-// the tree walk's where box_verdict leaves the question open (about one box in
-// a hundred). The walk is bound by instruction fetch: inline copies at each
-// site cost more than the calls.
+// the tree walk's where box_verdict leaves the question open. The walk is bound
+// by instruction fetch: inline copies at each site cost more than the calls.
 template <class WS>
 static __device__ __noinline__ bool box_in_table(const WS* ws, int owner, f3 lo, f3 hi) {
   const Cone c = load_cone(ws, owner);
@@ -696,7 +695,10 @@ static __device__ __noinline__ InOrder walk_in_order(const float4* __restrict__ 
 // the others wait until 32 are tested, and drawn, together: in a walk of each
 // node by the whole packet the projections and the hull took every lane's time
 // where a few needed them (prefiltered sky cones over 1 M triangles: 105 ->
-// 34 ms, light cones over 2 M: 33 -> 18.5 ms). A node splatted
+// 34 ms, light cones over 2 M: 33 -> 18.5 ms; meshes of a dozen triangles,
+// which have no nodes to share out, lose: 64 boxes under sky cones 1.74 ->
+// 2.02 ms, and walking such meshes in order gave 1.92 there but cost every
+// other scene 3 to 6 %). A node splatted
 // while its mesh is walked is an integer sum like a triangle's, so its order
 // does not matter either.
 template <bool kCount, class WS>
@@ -764,7 +766,10 @@ __device__ __forceinline__ void walk_splat_pairs(const DevScene& s, LaneState<WS
 // and tests both children. Within a mesh the order of the visits does not
 // matter: the accumulated areas are exact integers and no early-out looks at
 // them; only the cap does, and a cone whose work reaches it here is walked
-// again in order (walk_in_order), its accumulator cleared. A packet's cones
+// again in order (walk_in_order), its accumulator cleared: so calls with caps far
+// below the defaults lose (518,000 cones over 40 spheres, against the walk in
+// order alone: caps of 300 and 150 2.39 -> 3.38 ms, 1,000 and 512 3.79 -> 2.05,
+// the defaults 3.77 -> 1.90). A packet's cones
 // share few nodes below a mesh's first levels: walked as a union, 9 of 32
 // lanes were active in the box tests and a packet took 252 steps where its
 // cones needed 53 each.
